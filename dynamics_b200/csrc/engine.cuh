@@ -136,12 +136,12 @@ struct SysView {
     // columns
     uint32_t ncx, ncy, ncol;
     uint32_t ancx, ancy, ancol;   // a finer column grid for non-water atoms
-    uint32_t* col_count; uint32_t* col_off; uint32_t* col_fill;   // [ncol(+1)]
-    uint32_t* col_boff;                         // unpadded bucket offsets [ncol+1]
-    uint32_t* acol_count; uint32_t* acol_off; uint32_t* acol_fill; uint32_t* acol_boff;
-    uint32_t* wnew;                             // new slot of each old water slot
+    uint32_t* col_count; uint32_t* col_off;     // [ncol+1]
+    uint32_t* acol_count; uint32_t* acol_off;
+    uint32_t* wplace; uint32_t* aplace;         // place of each water / atom in its column's bucket
     float* wkey; float* akey;                   // z sort keys (fraction of the box)
-    uint32_t* bucket; uint32_t* abucket;        // unsorted column members
+    uint32_t* bucket; uint32_t* abucket;        // unsorted column members and their sort keys (z, index)
+    unsigned long long* bkey; unsigned long long* abkey;
     uint32_t* wcol; uint32_t* acol;             // column of each water / atom
     // cluster bounding boxes (center xyz, half extent xyz)
     float4* wbb_c; float4* wbb_h; float4* abb_c; float4* abb_h;
@@ -161,10 +161,9 @@ struct SysView {
     uint32_t union_chunk;         // waters staged in shared memory at a time
     uint32_t ww_split;            // CTAs sharing one group's list entries (small systems)
     float4* gbb_c; float4* gbb_h;
-    uint32_t* tile_n; uint32_t* tile_j;      // [ngrp_cap], [ngrp_cap*cap_tile]
+    uint32_t* tile_j;                        // [ngrp_cap*cap_tile] rebuild scratch
     uint32_t* grp_nrun; uint32_t* grp_nloc;  // [ngrp_cap]
     uint2* grp_run;                          // [ngrp_cap*cap_run] (slot, union offset)
-    uint16_t* cand_loc;                      // [ngrp_cap*cap_tile*8] rebuild scratch
     uint32_t* wnb_n; uint16_t* wnb;          // [nw_cap], [nw_cap*cap_nb]
     // the lists the water-water kernel walks: wnb pruned to molecule pairs
     // within r_in (k_ww_prune), re-pruned when a water has moved half of

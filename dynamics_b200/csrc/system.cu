@@ -282,7 +282,7 @@ void enqueue_forces(dyn_sys_s* h, bool force_rebuild) {
     const Target T{&v, nullptr, st};
     if (!force_rebuild) dyn::launch_displacement_check(T);
     dyn::launch_rebuild(T, force_rebuild);
-    dyn::launch_prune(T, force_rebuild);
+    if (!force_rebuild) dyn::launch_prune(T, false);  // a rebuild writes the pruned lists too
     dyn::launch_gather_atoms(T);
     dyn::launch_pairs(T, true);
     dyn::launch_pair14(T, true);
@@ -632,8 +632,9 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     TRY(dev_alloc(h, &v.wtmp, 10 * (size_t)v.nw_cap));
     TRY(dev_alloc(h, &v.wtmp_id, v.nw_cap));
     TRY(dev_alloc(h, &v.wrecip, 9 * (size_t)std::max(1u, v.nw)));
-    TRY(dev_alloc(h, &v.wnew, v.nw_cap));
+    TRY(dev_alloc(h, &v.wplace, v.nw_cap));
     TRY(dev_alloc(h, &v.wkey, v.nw_cap));
+    TRY(dev_alloc(h, &v.bkey, v.nw_cap));
     TRY(dev_alloc(h, &v.wcol, v.nw_cap));
     TRY(dev_alloc(h, &v.bucket, v.nw_cap));
     TRY(dev_alloc(h, &v.apos, std::max(1u, v.na)));
@@ -652,28 +653,24 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     TRYC(cudaMemsetAsync(v.sidx, 0xFF, v.na_cap * sizeof(uint32_t), h->stream));
     TRY(dev_alloc(h, &v.aslot, std::max(1u, v.na)));
     TRY(dev_alloc(h, &v.akey, std::max(1u, v.na)));
+    TRY(dev_alloc(h, &v.abkey, std::max(1u, v.na)));
+    TRY(dev_alloc(h, &v.aplace, std::max(1u, v.na)));
     TRY(dev_alloc(h, &v.acol, std::max(1u, v.na)));
     TRY(dev_alloc(h, &v.abucket, std::max(1u, v.na)));
     TRY(dev_alloc(h, &v.col_count, v.ncol + 1));
     TRY(dev_alloc(h, &v.col_off, v.ncol + 1));
-    TRY(dev_alloc(h, &v.col_fill, v.ncol + 1));
-    TRY(dev_alloc(h, &v.col_boff, v.ncol + 1));
     TRY(dev_alloc(h, &v.acol_count, v.ancol + 1));
     TRY(dev_alloc(h, &v.acol_off, v.ancol + 1));
-    TRY(dev_alloc(h, &v.acol_fill, v.ancol + 1));
-    TRY(dev_alloc(h, &v.acol_boff, v.ancol + 1));
     TRY(dev_alloc(h, &v.wbb_c, v.nwclus_cap));
     TRY(dev_alloc(h, &v.wbb_h, v.nwclus_cap));
     TRY(dev_alloc(h, &v.abb_c, v.naclus_cap));
     TRY(dev_alloc(h, &v.abb_h, v.naclus_cap));
     TRY(dev_alloc(h, &v.gbb_c, v.ngrp_cap));
     TRY(dev_alloc(h, &v.gbb_h, v.ngrp_cap));
-    TRY(dev_alloc(h, &v.tile_n, v.ngrp_cap));
     TRY(dev_alloc(h, &v.tile_j, (size_t)v.ngrp_cap * v.cap_tile));
     TRY(dev_alloc(h, &v.grp_nrun, v.ngrp_cap));
     TRY(dev_alloc(h, &v.grp_nloc, v.ngrp_cap));
     TRY(dev_alloc(h, &v.grp_run, (size_t)v.ngrp_cap * v.cap_run));
-    TRY(dev_alloc(h, &v.cand_loc, (size_t)v.ngrp_cap * v.cap_tile * WCL));
     TRY(dev_alloc(h, &v.wnb_n, v.nw_cap));
     TRY(dev_alloc(h, &v.wnb, (size_t)v.nw_cap * v.cap_nb));
     TRY(dev_alloc(h, &v.winb_n, v.nw_cap));
@@ -1306,12 +1303,9 @@ int count_step_kernels(dyn_sys_s* h, bool spme, uint32_t* fixed, uint32_t* rebui
         }
         *fixed = total - fft;
     }
-    // a rebuild is always followed by a prune of the water-water lists (which
-    // also runs alone, 2 kernels, when only the prune buffer is used up)
-    if (rebuild && (rc = count([&] {
-            dyn::launch_rebuild(T, false);
-            dyn::launch_prune(T, false);
-        }, rebuild))) return rc;
+    // a prune of the water-water lists runs alone (2 kernels, not counted
+    // here) when only the prune buffer is used up
+    if (rebuild && (rc = count([&] { dyn::launch_rebuild(T, false); }, rebuild))) return rc;
     if (periodic && (rc = count([&] { dyn::launch_periodic(T); }, periodic))) return rc;
     return DYN_OK;
 }

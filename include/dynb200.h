@@ -389,7 +389,7 @@ typedef struct {
     double dh_dl;             /* alchemical dH/dlambda, kcal/mol (short-range
                                * cross pairs + SPME cross term), energy steps */
     uint64_t list_prunes;     /* prunes of the water-water lists so far (every
-                               * rebuild is followed by one) */
+                               * rebuild includes one) */
 } dyn_energies_t;
 
 /* Creates a resident system (replaces MdState::new's device setup,
@@ -461,9 +461,9 @@ int dyn_sys_stage_times(dyn_sys_t h, uint32_t n_steps, float dt, double* ms);
  * (COM removal, recentering, reset_angle). */
 int dyn_sys_launches_per_step(dyn_sys_t h, int spme, uint32_t* out);
 
-/* Kernels a step adds when it rebuilds the lists (*rebuild, including the
- * prune of the water-water lists that follows every rebuild; a step that
- * only prunes adds 2) and when a periodic task is due (*periodic); in the
+/* Kernels a step adds when it rebuilds the lists (*rebuild; the rebuild
+ * writes the pruned water-water lists too; a step that only prunes adds 2)
+ * and when a periodic task is due (*periodic); in the
  * captured step graph these sit under conditional nodes that the device
  * sets. */
 int dyn_sys_launches_conditional(dyn_sys_t h, uint32_t* rebuild, uint32_t* periodic);
