@@ -4,8 +4,9 @@
 // kernel body as the single-system engine, in its NAME##_batch form, with a
 // block map that gives each system the block range its single-system launch
 // would have had (per-system offsets into one grid).  A step is one captured
-// CUDA graph whose list rebuild and periodic tasks sit under IF nodes that
-// any member can raise; each member's kernels still check its own flags, so
+// CUDA graph whose list rebuild and prune sit under a switch node that any
+// member can raise, with the periodic tasks launched after it when a member
+// is due; each member's kernels still check its own flags, so
 // a member's trajectory is bit-identical to running it alone.  cuFFT runs
 // once per member on the batch stream (its plans are per grid size).
 //
@@ -74,6 +75,7 @@ struct dyn_batch_s {
     std::vector<dyn_sys_t> members;
     BatchCtx ctx;
     SysView* d_views[4] = {nullptr, nullptr, nullptr, nullptr};  // one per graph variant
+    unsigned int* vote = nullptr;   // the members' votes on list work (SysView::bvote), zero between steps
     std::vector<void*> map_allocs;
     cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
     float graph_dt[4] = {0, 0, 0, 0};
@@ -123,38 +125,36 @@ int upload_maps(dyn_batch_s* b) {
 }
 
 // The stages of one step, for all members at once (MdState::step,
-// src/integrate.rs:100-473).  With cond, the rebuild and the periodic tasks
-// go under IF nodes of the capture in progress.
+// src/integrate.rs:100-473).  With cond, the rebuild and the prune are the
+// bodies of the capture's switch node; the rebuild's body prunes too, as one
+// member may need the one and another the other.
 int enqueue_batch_step(dyn_batch_s* b, float dt, bool spme, bool energy, bool cond,
-                       cudaGraphConditionalHandle c_rebuild, cudaGraphConditionalHandle c_prune,
-                       cudaGraphConditionalHandle c_periodic) {
+                       cudaGraphConditionalHandle c_lists) {
     const Target T{nullptr, &b->ctx, b->stream}, TA{nullptr, &b->ctx, b->aux};
     const Target S0{nullptr, &b->ctx, b->br.side[0]}, S1{nullptr, &b->ctx, b->br.side[1]};
-    cudaGraph_t body = nullptr;
     int rc = DYN_OK;
     // cond: capturing (parallel branches); otherwise a collecting pass
     if ((rc = dyn::enqueue_first_half(T, S0, b->br, cond, dt)) != DYN_OK) return rc;
-    dyn::launch_displacement_check(T);
-    if (cond && (rc = dyn::begin_if_body(b->stream, b->aux, c_rebuild, &body)) != DYN_OK) return rc;
+    cudaGraph_t body[2] = {};
+    if (cond && (rc = dyn::add_switch(b->stream, c_lists, body)) != DYN_OK) return rc;
+    if (cond && (rc = dyn::begin_body(b->aux, body[LISTS_REBUILD])) != DYN_OK) return rc;
     dyn::launch_rebuild(cond ? TA : T, false);
-    if (cond && (rc = dyn::end_if_body(b->aux)) != DYN_OK) return rc;
-    if (cond && (rc = dyn::begin_if_body(b->stream, b->aux, c_prune, &body)) != DYN_OK) return rc;
+    if (cond) dyn::launch_prune(TA, false);
+    if (cond && (rc = dyn::end_body(b->aux)) != DYN_OK) return rc;
+    if (cond && (rc = dyn::begin_body(b->aux, body[LISTS_PRUNE])) != DYN_OK) return rc;
     dyn::launch_prune(cond ? TA : T, false);
-    if (cond && (rc = dyn::end_if_body(b->aux)) != DYN_OK) return rc;
-    dyn::launch_gather_atoms(T);
+    if (cond && (rc = dyn::end_body(b->aux)) != DYN_OK) return rc;
     if ((rc = dyn::enqueue_forces(T, S0, S1, b->br, cond, spme, energy)) != DYN_OK) return rc;
     if ((rc = dyn::enqueue_second_half(T, S0, b->br, cond, dt)) != DYN_OK) return rc;
     dyn::launch_finalize(T, dt, energy, true);
-    if (cond && (rc = dyn::begin_if_body(b->stream, b->aux, c_periodic, &body)) != DYN_OK) return rc;
-    dyn::launch_periodic(cond ? TA : T);
-    if (cond && (rc = dyn::end_if_body(b->aux)) != DYN_OK) return rc;
+    if (!cond) dyn::launch_periodic(T);  // its block maps; launched after the graph when due
     return DYN_OK;
 }
 
 // Records the block maps of a step variant (no launches) and uploads them.
 int collect_maps(dyn_batch_s* b, float dt, bool spme, bool energy) {
     b->ctx.collecting = true;
-    const int rc = enqueue_batch_step(b, dt, spme, energy, false, 0, 0, 0);
+    const int rc = enqueue_batch_step(b, dt, spme, energy, false, 0);
     b->ctx.collecting = false;
     if (rc) return rc;
     return upload_maps(b);
@@ -181,17 +181,9 @@ int capture_batch_step(dyn_batch_s* b, int g, float dt, bool spme, bool energy, 
     b->ctx.d_views = b->d_views[g];
     b->ctx.map_missing = false;
     DYN_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    cudaGraphConditionalHandle hr = 0, hq = 0, hp = 0;
-    {
-        cudaStreamCaptureStatus cs;
-        cudaGraph_t cg = nullptr;
-        cudaError_t e = cudaStreamGetCaptureInfo(b->stream, &cs, nullptr, &cg, nullptr, nullptr);
-        if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hr, cg, 0, cudaGraphCondAssignDefault);
-        if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hq, cg, 0, cudaGraphCondAssignDefault);
-        if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hp, cg, 0, cudaGraphCondAssignDefault);
-        if (e != cudaSuccess) rc = dyn::cuda_fail(e, "cudaGraphConditionalHandleCreate");
-    }
-    if (rc == DYN_OK) rc = enqueue_batch_step(b, dt, spme, energy, true, hr, hq, hp);
+    cudaGraphConditionalHandle hl = 0;
+    rc = dyn::create_switch_handle(b->stream, &hl);
+    if (rc == DYN_OK) rc = enqueue_batch_step(b, dt, spme, energy, true, hl);
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
     if (rc == DYN_OK && e != cudaSuccess) rc = dyn::cuda_fail(e, "cudaStreamEndCapture");
@@ -205,12 +197,12 @@ int capture_batch_step(dyn_batch_s* b, int g, float dt, bool spme, bool energy, 
         return rc;
     }
     // the graph's kernels read the views at run time: give them this
-    // graph's conditional handles
+    // graph's switch handle
     for (SysView& v : b->ctx.views) {
-        v.cond_rebuild = hr;
-        v.cond_prune = hq;
-        v.cond_periodic = hp;
+        v.cond_lists = hl;
         v.use_cond = 1;
+        v.bvote = b->vote;
+        v.bmembers = (uint32_t)b->ctx.views.size();
     }
     const cudaError_t ue = cudaMemcpy(b->d_views[g], b->ctx.views.data(), b->ctx.views.size() * sizeof(SysView),
                                       cudaMemcpyHostToDevice);
@@ -231,6 +223,7 @@ extern "C" int dyn_batch_destroy(dyn_batch_t b) {
         if (b->graph[g]) cudaGraphExecDestroy(b->graph[g]);
         if (b->d_views[g]) cudaFree(b->d_views[g]);
     }
+    if (b->vote) cudaFree(b->vote);
     for (void* p : b->map_allocs) cudaFree(p);
     for (dyn_sys_t m : b->members) dyn_sys_destroy(m);
     if (b->io.d_state) cudaFree(b->io.d_state);
@@ -281,6 +274,9 @@ extern "C" int dyn_batch_create(void* stream, uint32_t n, const dyn_config_t* cf
             if (e2 != cudaSuccess) { dyn_batch_destroy(b); return dyn::cuda_fail(e2, "cudaEventCreateWithFlags"); }
         }
         b->ctx.n_fft = BatchCtx::N_FFT;
+        cudaError_t e3 = cudaMalloc(&b->vote, 2 * sizeof(unsigned int));
+        if (e3 == cudaSuccess) e3 = cudaMemset(b->vote, 0, 2 * sizeof(unsigned int));
+        if (e3 != cudaSuccess) { dyn_batch_destroy(b); return dyn::cuda_fail(e3, "cudaMalloc (batch votes)"); }
     }
     if (n > 0) {
         b->spme_interval = std::max(1u, cfgs[0].spme_interval);
@@ -323,7 +319,17 @@ extern "C" int dyn_batch_step(dyn_batch_t b, uint32_t n_steps, float dt) {
         }
         DYN_CUDA(cudaGraphLaunch(b->graph[g], b->stream));
         b->host_step += 1;
-        for (dyn_sys_t m : b->members) m->host_step += 1;
+        bool due = false;
+        for (dyn_sys_t m : b->members) {
+            m->host_step += 1;
+            due = due || dyn::periodic_due(m->v, m->host_step);
+        }
+        if (due) {
+            // the members' kernels check their own step numbers
+            b->ctx.d_views = b->d_views[g];
+            dyn::launch_periodic(Target{nullptr, &b->ctx, b->stream});
+            DYN_CUDA(cudaGetLastError());
+        }
         // at most about 2 x 512 steps queued at a time
         if ((i + 1) % 512 == 0 && i + 1 < n_steps) {
             if (!b->window_ev) DYN_CUDA(cudaEventCreateWithFlags(&b->window_ev, cudaEventDisableTiming));
@@ -375,7 +381,7 @@ extern "C" int dyn_batch_launches(dyn_batch_t b, int spme, uint32_t* fixed, uint
         b->ctx.collecting = false;
         return b->ctx.launches;
     };
-    const uint32_t all = count([&] { enqueue_batch_step(b, 0.002f, spme != 0, true, false, 0, 0, 0); });
+    const uint32_t all = count([&] { enqueue_batch_step(b, 0.002f, spme != 0, true, false, 0); });
     *rebuild = count([&] { dyn::launch_rebuild(T, false); });
     const uint32_t prune = count([&] { dyn::launch_prune(T, false); });
     *periodic = count([&] { dyn::launch_periodic(T); });

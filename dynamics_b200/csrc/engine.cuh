@@ -240,11 +240,15 @@ struct SysView {
     // float32)
     float poly_g[NPOLY_G];
     float two_over_rc2;
-    // IF-node handles of the captured step graph: the displacement check
-    // sets cond_rebuild, the step finalisation sets cond_periodic; only
-    // kernels captured for a graph (use_cond != 0) set them
-    cudaGraphConditionalHandle cond_rebuild, cond_periodic, cond_prune;
-    uint32_t use_cond;
+    // switch-node handle of the captured step graph, set by the displacement
+    // check to LISTS_REBUILD or LISTS_PRUNE where the lists need it; only
+    // kernels captured for a graph (use_cond != 0) set it.  In a batch every
+    // member votes into bvote ({members done, union of their wishes}) and
+    // the last of the bmembers sets the node.
+    cudaGraphConditionalHandle cond_lists;
+    uint32_t use_cond, bmembers;
+    unsigned int* bvote;
+    uint32_t first_blocks;  // blocks of the first-half kernels, which vote on the displacements
     uint32_t nb[NREGION];   // blocks each region's kernel is launched with
     int plan_f, plan_b;     // cuFFT plans (host-side handles, used by launch code only)
 };
@@ -268,6 +272,55 @@ struct Blk { uint32_t idx, cnt; };
 // (measured on the step graphs).
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Bodies of the step graph's switch node (any other value: neither).
+enum ListWork { LISTS_REBUILD = 0, LISTS_PRUNE = 1, LISTS_KEEP = 2 };
+
+// The displacement check (src/neighbors.rs:159-169): a block's largest squared
+// displacements since the last rebuild (m) and prune (mp) go to the system's
+// maxima, and the last of total blocks decides: rebuild when a molecule has
+// moved half the buffer, else prune when a water has moved half the inner
+// buffer (the rebuild writes the pruned lists too).
+__device__ __forceinline__ void displacement_vote(const SysView& v, float m, float mp, uint32_t total) {
+    __shared__ float sm[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    m = warp_max_f(m);
+    mp = warp_max_f(mp);
+    if (lane == 0) { sm[0][w] = m; sm[1][w] = mp; }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (uint32_t k = 1; k < blockDim.x >> 5; ++k) { m = fmaxf(m, sm[0][k]); mp = fmaxf(mp, sm[1][k]); }
+    Scalars* sc = v.sc;
+    if (m > 0.f) atomicMax(&sc->max_disp2_bits, __float_as_uint(m));
+    if (mp > 0.f) atomicMax(&sc->max_dprune_bits, __float_as_uint(mp));
+    __threadfence();
+    if (atomicAdd(&sc->ctr_disp, 1u) != total - 1) return;
+    __threadfence();
+    const float mx = __uint_as_float(atomicExch(&sc->max_disp2_bits, 0u));
+    const float mxp = __uint_as_float(atomicExch(&sc->max_dprune_bits, 0u));
+    const float h = 0.5f * v.buffer, hp = 0.5f * v.prune_buf;
+    const bool need = sc->need_rebuild || mx >= h * h;
+    const bool need_p = !need && (sc->need_prune || mxp >= hp * hp);
+    sc->need_rebuild = need ? 1u : 0u;
+    sc->need_prune = need_p ? 1u : 0u;
+    if (mx >= 1e29f || mxp >= 1e29f) sc->nonfinite = 1u;
+    sc->ctr_disp = 0u;
+    if (!v.use_cond) return;
+    bool rebuild = need, prune = need_p;
+    if (v.bvote) {
+        const unsigned int wish = (need ? 1u : 0u) | (need_p ? 2u : 0u);
+        if (wish) atomicOr(&v.bvote[1], wish);
+        __threadfence();
+        if (atomicAdd(&v.bvote[0], 1u) != v.bmembers - 1) return;
+        __threadfence();
+        const unsigned int all = atomicExch(&v.bvote[1], 0u);
+        v.bvote[0] = 0u;
+        rebuild = all & 1u;
+        prune = all & 2u;
+    }
+    if (rebuild) cudaGraphSetConditional(v.cond_lists, LISTS_REBUILD);
+    else if (prune) cudaGraphSetConditional(v.cond_lists, LISTS_PRUNE);
 }
 
 #define DYN_UNPAREN(...) __VA_ARGS__
@@ -448,6 +501,9 @@ void launch_second_half_water(const Target& t, float dt);
 void launch_second_half_atoms(const Target& t, float dt);
 void launch_finalize(const Target& t, float dt, bool energy, bool thermo);
 void launch_periodic(const Target& t);
+// whether the periodic tasks have work after step number next: COM removal,
+// recentering, reset_angle or a snapshot
+bool periodic_due(const SysView& v, uint64_t next);
 void launch_bonded(const Target& t, bool energy);
 int kick_blocks_w(const SysView& v);
 int kick_blocks_a(const SysView& v);

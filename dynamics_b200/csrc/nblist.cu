@@ -15,7 +15,7 @@
 //      below cutoff + twice the O-H reach + buffer).
 // Every kernel of the rebuild returns immediately unless the displacement
 // check raised Scalars::need_rebuild; inside a captured step graph the
-// rebuild kernels also sit under a conditional (IF) node that the check
+// rebuild kernels also sit under a conditional (switch) node that the check
 // sets, so steps without a rebuild launch none of them.  The rebuild criterion is the reference's: max displacement since
 // the last rebuild >= buffer / 2 (src/neighbors.rs:159-169), tracking water
 // O only (src/neighbors.rs:71-82); water list radii add twice the O-H reach.
@@ -51,7 +51,8 @@ __device__ __forceinline__ uint32_t column_of(float3 p, const BoxDev& b, uint32_
 }
 
 // ---------------------------------------------------------------------------
-// displacement check
+// displacement check of an evaluation without a step; a step's first half
+// checks as it moves (integrate.cu)
 // ---------------------------------------------------------------------------
 DYN_KERNEL(, k_disp_check, (), ()) {
     const BoxDev b = *v.box;
@@ -74,32 +75,7 @@ DYN_KERNEL(, k_disp_check, (), ()) {
         const float d2 = dot3(d, d);
         m = fmaxf(m, isfinite(d2) ? d2 : 1e30f);
     }
-    m = warp_max_f(m);
-    mp = warp_max_f(mp);
-    if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(&v.sc->max_disp2_bits, __float_as_uint(m));
-    if ((threadIdx.x & 31) == 0 && mp > 0.f) atomicMax(&v.sc->max_dprune_bits, __float_as_uint(mp));
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    if (atomicAdd(&v.sc->ctr_disp, 1u) != bk.cnt - 1) return;
-    // the last block to finish sees every block's maximum and decides:
-    // rebuild when the largest displacement reaches half the buffer
-    __threadfence();
-    const float mx = __uint_as_float(atomicExch(&v.sc->max_disp2_bits, 0u));
-    const float mxp = __uint_as_float(atomicExch(&v.sc->max_dprune_bits, 0u));
-    const float h = 0.5f * v.buffer;
-    unsigned int need = v.sc->need_rebuild;
-    if (mx >= h * h) need = 1u;
-    v.sc->need_rebuild = need;
-    // a rebuild writes the pruned lists too; otherwise prune when a water has
-    // moved half the inner buffer
-    const float hp = 0.5f * v.prune_buf;
-    const unsigned int need_p = !need && (v.sc->need_prune || mxp >= hp * hp) ? 1u : 0u;
-    v.sc->need_prune = need_p;
-    if (mx >= 1e29f || mxp >= 1e29f) v.sc->nonfinite = 1u;
-    v.sc->ctr_disp = 0u;
-    if (v.use_cond && need) cudaGraphSetConditional(v.cond_rebuild, 1u);
-    if (v.use_cond && need_p) cudaGraphSetConditional(v.cond_prune, 1u);
+    displacement_vote(v, m, mp, bk.cnt);
 }
 
 // ---------------------------------------------------------------------------
@@ -843,7 +819,8 @@ DYN_KERNEL(, k_rebuild_done, (, bool force), (, force)) {
 }
 
 // Copies positions into cluster order and zeroes the atoms' and the
-// waters' short-range force accumulators (every pair kernel adds to them).
+// waters' short-range force accumulators (every pair kernel adds to them),
+// for an evaluation without a step; a step's first half does both.
 DYN_KERNEL(, k_gather_atoms, (), ()) {
     const uint32_t t0 = bk.idx * blockDim.x + threadIdx.x, stride = bk.cnt * blockDim.x;
     for (uint32_t s = t0; s < v.na_cap; s += stride) {

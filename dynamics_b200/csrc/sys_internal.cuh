@@ -110,10 +110,13 @@ void set_ww_split(dyn_sys_s* h, uint32_t split);
 // computes alone.
 void set_batch_member(dyn_sys_s* h);
 
-// Inside an active capture on st: appends an IF node on hc after everything
-// captured so far and starts capturing its body on aux.
-int begin_if_body(cudaStream_t st, cudaStream_t aux, cudaGraphConditionalHandle hc, cudaGraph_t* body);
-int end_if_body(cudaStream_t aux);
+// Inside an active capture on st: makes the handle of the step's switch node
+// (LISTS_KEEP at every launch); appends the node, with two bodies, after
+// everything captured so far; captures a body on aux.
+int create_switch_handle(cudaStream_t st, cudaGraphConditionalHandle* hc);
+int add_switch(cudaStream_t st, cudaGraphConditionalHandle hc, cudaGraph_t (&body)[2]);
+int begin_body(cudaStream_t aux, cudaGraph_t body);
+int end_body(cudaStream_t aux);
 // Copies the scalars to the host and turns device-side flags into errors.
 int read_scalars(dyn_sys_s* h);
 // Kernel nodes of a graph (library kernels included).

@@ -10,9 +10,7 @@
 
 #include "sys_internal.cuh"
 
-using dyn::begin_if_body;
 using dyn::count_graph_kernels;
-using dyn::end_if_body;
 using dyn::read_scalars;
 
 namespace {
@@ -112,16 +110,14 @@ void set_block_counts(SysView& v) {
     v.nb[REG_PME] = dyn::pme_blocks(v);
     v.nb[REG_CORR] = dyn::gather_blocks(v);
     v.nb[REG_CORR_A] = dyn::corr_blocks(v);
+    v.first_blocks = (v.nw ? dyn::kick_blocks_w(v) : 0) + v.nb[REG_CONS];
     v.nb[REG_COM] = dyn::kick_blocks_w(v) > dyn::kick_blocks_a(v) ? dyn::kick_blocks_w(v)
                                                                    : dyn::kick_blocks_a(v);
 }
 
-// Inside an active capture on st: appends an IF node on hc after everything
-// captured so far (later work depends on it) and starts capturing its body
-// on aux.
 }  // namespace
 namespace dyn {
-int begin_if_body(cudaStream_t st, cudaStream_t aux, cudaGraphConditionalHandle hc, cudaGraph_t* body) {
+int add_switch(cudaStream_t st, cudaGraphConditionalHandle hc, cudaGraph_t (&body)[2]) {
     cudaStreamCaptureStatus cs;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -129,23 +125,30 @@ int begin_if_body(cudaStream_t st, cudaStream_t aux, cudaGraphConditionalHandle 
     DYN_CUDA(cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, &deps, &nd));
     cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
     cp.conditional.handle = hc;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
+    cp.conditional.type = cudaGraphCondTypeSwitch;
+    cp.conditional.size = 2;
     cudaGraphNode_t node;
     DYN_CUDA(cudaGraphAddNode(&node, cg, deps, nd, &cp));
     DYN_CUDA(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-    *body = cp.conditional.phGraph_out[0];
-    DYN_CUDA(cudaStreamBeginCaptureToGraph(aux, *body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    body[0] = cp.conditional.phGraph_out[0];
+    body[1] = cp.conditional.phGraph_out[1];
     return DYN_OK;
 }
-}  // namespace dyn
-namespace {
-
-}  // namespace
-namespace dyn {
-int end_if_body(cudaStream_t aux) {
+int begin_body(cudaStream_t aux, cudaGraph_t body) {
+    DYN_CUDA(cudaStreamBeginCaptureToGraph(aux, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    return DYN_OK;
+}
+int end_body(cudaStream_t aux) {
     cudaGraph_t g = nullptr;
     DYN_CUDA(cudaStreamEndCapture(aux, &g));
+    return DYN_OK;
+}
+
+int create_switch_handle(cudaStream_t st, cudaGraphConditionalHandle* hc) {
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t cg = nullptr;
+    DYN_CUDA(cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, nullptr, nullptr));
+    DYN_CUDA(cudaGraphConditionalHandleCreate(hc, cg, LISTS_KEEP, cudaGraphCondAssignDefault));
     return DYN_OK;
 }
 
@@ -211,13 +214,14 @@ void Branches::destroy() {
 namespace {
 
 // Captures one step (MdState::step, src/integrate.rs:100-473) into a graph.
-// The list rebuild and the periodic tasks (COM removal, recentering,
-// reset_angle) sit under IF nodes that the displacement check and the step
-// finalisation set on the device, so a step that needs neither launches none
-// of their kernels.  body_rebuild / body_periodic receive the bodies (owned
-// by *out).
-int capture_step(dyn_sys_s* h, float dt, bool spme, bool energy, cudaGraph_t* out,
-                 cudaGraph_t* body_rebuild = nullptr, cudaGraph_t* body_periodic = nullptr) {
+// The list rebuild and the prune are the two bodies of one switch node that
+// the displacement check sets on the device, so a step that needs neither
+// launches none of their kernels.  A conditional node that does not fire
+// still costs about 5 us between the kernels around it (measured on the step
+// graphs), so there is one and not one each; the periodic tasks (COM
+// removal, recentering, reset_angle, snapshots) depend on the step number
+// only, which the host knows, and are launched after the graph when due.
+int capture_step(dyn_sys_s* h, float dt, bool spme, bool energy, cudaGraph_t* out) {
     SysView& v = h->v;
     cudaStream_t st = h->stream;
     const Target T{&v, nullptr, st};
@@ -226,35 +230,21 @@ int capture_step(dyn_sys_s* h, float dt, bool spme, bool energy, cudaGraph_t* ou
     *out = nullptr;
     DYN_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int rc = DYN_OK;
-    cudaGraph_t br = nullptr, bp = nullptr;
     do {
-        cudaStreamCaptureStatus cs;
-        cudaGraph_t cg = nullptr;
-        cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &cg, nullptr, nullptr);
-        if (e == cudaSuccess)
-            e = cudaGraphConditionalHandleCreate(&v.cond_rebuild, cg, 0, cudaGraphCondAssignDefault);
-        if (e == cudaSuccess)
-            e = cudaGraphConditionalHandleCreate(&v.cond_periodic, cg, 0, cudaGraphCondAssignDefault);
-        if (e == cudaSuccess)
-            e = cudaGraphConditionalHandleCreate(&v.cond_prune, cg, 0, cudaGraphCondAssignDefault);
-        if (e != cudaSuccess) { rc = dyn::cuda_fail(e, "cudaGraphConditionalHandleCreate"); break; }
+        if ((rc = dyn::create_switch_handle(st, &v.cond_lists)) != DYN_OK) break;
         v.use_cond = 1;
         if ((rc = dyn::enqueue_first_half(T, S0, h->br, true, dt)) != DYN_OK) break;
-        dyn::launch_displacement_check(T);
-        if ((rc = begin_if_body(st, h->aux, v.cond_rebuild, &br)) != DYN_OK) break;
+        cudaGraph_t body[2];
+        if ((rc = dyn::add_switch(st, v.cond_lists, body)) != DYN_OK) break;
+        if ((rc = dyn::begin_body(h->aux, body[LISTS_REBUILD])) != DYN_OK) break;
         dyn::launch_rebuild(TA, false);
-        if ((rc = end_if_body(h->aux)) != DYN_OK) break;
-        cudaGraph_t bpr = nullptr;
-        if ((rc = begin_if_body(st, h->aux, v.cond_prune, &bpr)) != DYN_OK) break;
+        if ((rc = dyn::end_body(h->aux)) != DYN_OK) break;
+        if ((rc = dyn::begin_body(h->aux, body[LISTS_PRUNE])) != DYN_OK) break;
         dyn::launch_prune(TA, false);
-        if ((rc = end_if_body(h->aux)) != DYN_OK) break;
-        dyn::launch_gather_atoms(T);
+        if ((rc = dyn::end_body(h->aux)) != DYN_OK) break;
         if ((rc = dyn::enqueue_forces(T, S0, S1, h->br, true, spme, energy)) != DYN_OK) break;
         if ((rc = dyn::enqueue_second_half(T, S0, h->br, true, dt)) != DYN_OK) break;
         dyn::launch_finalize(T, dt, energy, true);
-        if ((rc = begin_if_body(st, h->aux, v.cond_periodic, &bp)) != DYN_OK) break;
-        dyn::launch_periodic(TA);
-        if ((rc = end_if_body(h->aux)) != DYN_OK) break;
     } while (0);
     v.use_cond = 0;
     cudaGraph_t g = nullptr;
@@ -269,8 +259,6 @@ int capture_step(dyn_sys_s* h, float dt, bool spme, bool energy, cudaGraph_t* ou
         return rc;
     }
     *out = g;
-    if (body_rebuild) *body_rebuild = br;
-    if (body_periodic) *body_periodic = bp;
     return DYN_OK;
 }
 
@@ -916,6 +904,10 @@ extern "C" int dyn_sys_step(dyn_sys_t h, uint32_t n_steps, float dt) {
         }
         DYN_CUDA(cudaGraphLaunch(h->graph[g], h->stream));
         h->host_step += 1;
+        if (dyn::periodic_due(h->v, h->host_step)) {
+            dyn::launch_periodic(Target{&h->v, nullptr, h->stream});
+            DYN_CUDA(cudaGetLastError());
+        }
         // at most about 2 x STEP_WINDOW steps queued at a time: every
         // STEP_WINDOW launches wait for the mark set STEP_WINDOW launches ago
         if ((i + 1) % STEP_WINDOW == 0 && i + 1 < n_steps) {
@@ -1202,11 +1194,9 @@ extern "C" int dyn_sys_stage_times(dyn_sys_t h, uint32_t n_steps, float dt, doub
         cudaEventRecord(ev[0], st);
         dyn::launch_first_half(T, dt);
         cudaEventRecord(ev[1], st);
-        dyn::launch_displacement_check(T);
         dyn::launch_rebuild(T, false);
         dyn::launch_prune(T, false);
         cudaEventRecord(ev[2], st);
-        dyn::launch_gather_atoms(T);
         dyn::launch_pairs_ww(T, energy);
         cudaEventRecord(ev[7], st);
         dyn::launch_pairs_ws(T, energy);
@@ -1237,7 +1227,7 @@ extern "C" int dyn_sys_stage_times(dyn_sys_t h, uint32_t n_steps, float dt, doub
         DYN_CUDA(cudaGetLastError());
         DYN_CUDA(cudaEventSynchronize(ev[6]));
         for (int k = 0; k < 6; ++k) acc[k] += el(k, k + 1);
-        acc[6] += el(2, 7);   // includes the force zeroing and the atoms' cluster-order copy before it
+        acc[6] += el(2, 7);
         acc[7] += el(7, 8);
         acc[8] += el(8, 3);
         if (spme && !alch) {
@@ -1279,8 +1269,6 @@ int count_step_kernels(dyn_sys_s* h, bool spme, uint32_t* fixed, uint32_t* rebui
         uint32_t total = 0, fft = 0;
         rc = count([&] {
             dyn::launch_first_half(T, 0.002f);
-            dyn::launch_displacement_check(T);
-            dyn::launch_gather_atoms(T);
             dyn::launch_pairs(T, true);
             dyn::launch_pair14(T, true);
             dyn::launch_bonded(T, true);

@@ -444,12 +444,11 @@ int dyn_sys_step_host(dyn_sys_t h, uint32_t n_steps, float dt, const float* atom
  * timers (ComputationTimeSums, src/util.rs:111-180): runs n_steps steps
  * without graphs, with CUDA events between stages on the handle's stream,
  * and writes the mean milliseconds per step of each stage into
- * ms[DYN_STAGES]: [0] first half (kick/drift/thermostat), [1] displacement
- * check, list rebuild and prune, [2] short-range pair kernels, [3] 1-4 and
+ * ms[DYN_STAGES]: [0] first half (kick/drift/thermostat and the
+ * displacement check), [1] list rebuild and prune, [2] short-range pair kernels, [3] 1-4 and
  * bonded terms, [4] SPME (mean over the steps that ran it), [5] kick,
  * reductions, thermostat/barostat and periodic tasks; the pair stage split
- * into [6] water-water (with the force zeroing and the atoms'
- * cluster-order copy before it), [7] water-atom, [8] atom-atom; the SPME
+ * into [6] water-water, [7] water-atom, [8] atom-atom; the SPME
  * stage (per SPME step, without an alchemical molecule) into [9] spread,
  * [10] FFTs and convolution, [11] gather, [12] corrections. */
 #define DYN_STAGES 13
@@ -464,8 +463,8 @@ int dyn_sys_launches_per_step(dyn_sys_t h, int spme, uint32_t* out);
 /* Kernels a step adds when it rebuilds the lists (*rebuild; the rebuild
  * writes the pruned water-water lists too; a step that only prunes adds 2)
  * and when a periodic task is due (*periodic); in the
- * captured step graph these sit under conditional nodes that the device
- * sets. */
+ * captured step graph the former sit under a conditional node that the device
+ * sets, and the latter are launched after the graph. */
 int dyn_sys_launches_conditional(dyn_sys_t h, uint32_t* rebuild, uint32_t* periodic);
 
 /* The pairs the resident engine's pair kernels evaluate at this moment, as
