@@ -28,11 +28,12 @@
 #define GRPW 32           // waters per i-group of the water-water kernel (4 clusters)
 #define NPOLY_G 14        // coefficients of the screened-Coulomb force polynomial (14: the virial within 1e-5 of float64)
 #define UMAX 5            // atoms per constraint unit (a heavy atom and up to 4 H)
-#define LPW 8             // lanes per i-water in the water-water kernel
+#define WW_CHUNK_BYTES (4 * 16 + 13 * 4 + 4)  // shared memory per staged water: sites, j sums, slot
 #define ACL 8             // atoms per cluster
 #define INVALID_ID 0xFFFFFFFFu
 #define PME_BRICK 8       // edge of the SPME grid bricks (grid points)
 #define DYN_SITE_WATER 0x80000000u  // site code flag: a water site (3 * id + site) rather than an atom
+#define WW_SPLIT_MAX 8    // most parts of a group's union in the water-water kernel
 #define WW_JFIX_SHIFT 16  // j-side water-water sums: int32 fixed point, 2^-16 kcal/mol/A
 #define NACC 16           // accumulator slots
 
@@ -52,8 +53,6 @@ struct Scalars {
     unsigned int overflow;        // largest list length that did not fit (0 = ok)
     unsigned int nonfinite;       // set when a kernel saw NaN/Inf
     unsigned int max_disp2_bits;  // float bits, atomicMax over non-negative floats
-    unsigned int timeout;         // a bounded device wait gave up
-    unsigned int pad1;
     double acc[NACC];             // finalised accumulators of the last step
     double recip_cache[4];        // e_recip, vir_recip, e_corr, vir_corr of last SPME step
     double csvr_lambda;
@@ -102,6 +101,14 @@ struct SiteRec {
 enum Region {
     REG_WW = 0, REG_WS, REG_SW, REG_SS, REG_14, REG_BOND, REG_KICK_W, REG_KICK_A,
     REG_CONS, REG_PME, REG_CORR, REG_CORR_A, REG_COM, NREGION
+};
+
+// What the pair kernels need of the interaction.  Screened-Coulomb force
+// q q (r^-3 + g(r^2)) d: g as a polynomial in t = 2 r^2 / rc^2 - 1 (Chebyshev
+// interpolation, power basis, Horner in float32).
+struct PairParams {
+    float poly_g[NPOLY_G];
+    float two_over_rc2, rc2, ljc2, alpha;
 };
 
 // Pointers and sizes passed by value to every kernel.
@@ -154,21 +161,20 @@ struct SysView {
     uint2* ws_item; uint2* ss_item;
     uint32_t ws_item_cap, ss_item_cap;
     // water-water: per 32-water i-group the candidate j-clusters (tile_j),
-    // the union of the waters its members need, stored as runs of
-    // consecutive slots (staged in shared memory by bulk copies), and per
-    // i-water a list of indices into that union
-    uint32_t ngrp_cap, cap_tile, cap_nb, cap_union, cap_run;
+    // the union of the waters its members need (staged in shared memory by
+    // asynchronous copies), and per i-water a list of indices into that union
+    uint32_t ngrp_cap, cap_tile, cap_nb, cap_union;
     uint32_t union_chunk;         // waters staged in shared memory at a time
-    uint32_t ww_split;            // CTAs sharing one group's list entries (small systems)
+    uint32_t ww_split;            // equal ranges of a group's union, a unit of work each
     float4* gbb_c; float4* gbb_h;
     uint32_t* tile_j;                        // [ngrp_cap*cap_tile] rebuild scratch
-    uint32_t* grp_nrun; uint32_t* grp_nloc;  // [ngrp_cap]
-    uint2* grp_run;                          // [ngrp_cap*cap_run] (slot, union offset)
+    uint32_t* grp_nloc;                      // [ngrp_cap]
     uint32_t* wnb_n; uint16_t* wnb;          // [nw_cap], [nw_cap*cap_nb]
     // the lists the water-water kernel walks: wnb pruned to molecule pairs
     // within r_in (k_ww_prune), re-pruned when a water has moved half of
     // r_in's buffer since the last prune (O positions then: wprune)
     uint32_t* winb_n; uint16_t* winb;        // [nw_cap], [nw_cap*cap_nb]
+    uint16_t* winb_cut;                      // [nw_cap*WW_SPLIT_MAX] first entry of each part (ww_split > 1)
     float4* wprune;                          // [nw_cap]
     uint32_t* grp_uslot;                     // [ngrp_cap*cap_union] union index -> slot
     // The molecule lists are half lists (each water pair once, listed by
@@ -212,7 +218,7 @@ struct SysView {
     double* partials;       // [NREGION][max_blocks][4]
     uint32_t max_blocks;
     // parameters
-    float rc, rc2, ljc2, alpha, buffer;
+    float rc, alpha, buffer;
     float r_ww, r_ws, r_ss;     // list radii
     float r_ws_skip2;           // (cutoff + O-H reach)^2: water-atom entries beyond it are skipped
     float r_in, prune_buf;      // pruned water-water radius and its buffer
@@ -235,11 +241,7 @@ struct SysView {
     uint32_t alch_on, alch_lo, alch_hi;
     float alch_cs, alch_dcs, alch_ll, alch_dll;
     double e_self;          // Ewald self energy -alpha/sqrt(pi) sum q^2
-    // screened-Coulomb force q q (r^-3 + g(r^2)) d: g as a polynomial in
-    // t = 2 r^2 / rc^2 - 1 (Chebyshev interpolation, power basis, Horner in
-    // float32)
-    float poly_g[NPOLY_G];
-    float two_over_rc2;
+    PairParams pp;
     // switch-node handle of the captured step graph, set by the displacement
     // check to LISTS_REBUILD or LISTS_PRUNE where the lists need it; only
     // kernels captured for a graph (use_cond != 0) set it.  In a batch every
@@ -273,6 +275,10 @@ struct Blk { uint32_t idx, cnt; };
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+
+// First union entry of part p of a group's union of n waters (the water-water
+// kernel's units of work).
+__device__ __forceinline__ uint32_t ww_cut(uint32_t n, uint32_t p, uint32_t split) { return n * p / split; }
 
 // Bodies of the step graph's switch node (any other value: neither).
 enum ListWork { LISTS_REBUILD = 0, LISTS_PRUNE = 1, LISTS_KEEP = 2 };

@@ -33,31 +33,22 @@ int d2h(std::vector<T>& out, const T* src, size_t n) {
 // water-water: the molecule pairs (i, j) the water-water kernel evaluates
 int ww_pairs(const SysView& v, const Scalars& sc, std::vector<uint32_t>& out) {
     const uint32_t ng = (sc.n_wclus + GRPW / WCL - 1) / (GRPW / WCL);
-    std::vector<uint32_t> wid, nloc, nrun, nb_n;
-    std::vector<uint2> runs;
+    std::vector<uint32_t> wid, nloc, uslot, nb_n;
     std::vector<uint16_t> nb;
     TRY_D2H(wid, v.wid, v.nw_cap);
     TRY_D2H(nloc, v.grp_nloc, ng);
-    TRY_D2H(nrun, v.grp_nrun, ng);
-    TRY_D2H(runs, v.grp_run, (size_t)ng * v.cap_run);
+    TRY_D2H(uslot, v.grp_uslot, (size_t)ng * v.cap_union);
     // the pruned lists: what the water-water kernel walks
     TRY_D2H(nb_n, v.winb_n, v.nw_cap);
     TRY_D2H(nb, v.winb, (size_t)v.nw_cap * v.cap_nb);
-    std::vector<uint32_t> uni;
     for (uint32_t g = 0; g < ng; ++g) {
-        // the group's union: union index -> slot, from its runs
-        uni.assign(nloc[g], INVALID_ID);
-        for (uint32_t t = 0; t < nrun[g]; ++t) {
-            const uint2 r = runs[(size_t)g * v.cap_run + t];
-            const uint32_t end = t + 1 < nrun[g] ? runs[(size_t)g * v.cap_run + t + 1].y : nloc[g];
-            for (uint32_t u = r.y; u < end && u < nloc[g]; ++u) uni[u] = r.x + (u - r.y);
-        }
+        const uint32_t* uni = uslot.data() + (size_t)g * v.cap_union;  // union index -> slot
         for (uint32_t il = 0; il < GRPW; ++il) {
             const uint32_t s = g * GRPW + il;
             if (s >= v.nw_cap || wid[s] == INVALID_ID) continue;
             for (uint32_t k = 0; k < nb_n[s]; ++k) {
                 const uint32_t u = nb[(size_t)s * v.cap_nb + k];
-                const uint32_t sj = u < uni.size() ? uni[u] : INVALID_ID;
+                const uint32_t sj = u < nloc[g] ? uni[u] : INVALID_ID;
                 if (sj == INVALID_ID || sj >= v.nw_cap || wid[sj] == INVALID_ID) continue;
                 out.push_back(wid[s]);
                 out.push_back(wid[sj]);

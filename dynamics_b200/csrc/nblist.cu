@@ -551,16 +551,15 @@ DYN_KERNEL(__launch_bounds__(IT_T), k_items, (, bool force), (, force)) {
 }
 
 // The candidate clusters of a water group, the union of the waters its
-// members need (as runs of consecutive slots), and per i-water lists of
-// indices into that union, in one pass; one CTA (256 threads) per group.
+// members need, and per i-water lists of indices into that union, in one
+// pass; one CTA (256 threads) per group.
 // Candidates: clusters within the list radius of the group's box, ascending;
 // the molecule lists are half lists (a pair belongs to its lower slot), so
 // only clusters from the group's own first on can hold a partner.  Each
 // candidate water is then tested against all 32 members, giving two 32-bit
 // masks: members within r_ww (the outer lists wnb) and within r_in (the
 // pruned lists winb).  A candidate with any member is in the union; the
-// needed ones are numbered with a block-wide scan, and a needed water whose
-// predecessor is not needed, or not the slot before, starts a run.  A warp
+// needed ones are numbered with a block-wide scan.  A warp
 // compacts the lists of four members from the masks with one ballot per 32
 // candidates, so every list ascends.  Everything is deterministic.
 // Bound by the distance tests, 32 per candidate: 24,000 waters in 98 A, 73 us,
@@ -578,10 +577,9 @@ DYN_KERNEL(__launch_bounds__(UT), k_group_union, (, bool force), (, force)) {
     const int tid = threadIdx.x, lane = tid & 31, wid_ = tid >> 5;
     constexpr int NWP = UT / 32, MPW = GRPW / NWP;  // warps, members per warp
     __shared__ float4 io[GRPW];
-    __shared__ uint32_t wt[TU][NWP], wn[NWP], wr[NWP];
-    __shared__ uint32_t sh_out[UT], sh_in[UT], sh_slot[UT];
+    __shared__ uint32_t wt[TU][NWP], wn[NWP];
+    __shared__ uint32_t sh_out[UT], sh_in[UT];
     __shared__ uint16_t sh_loc[UT];
-    __shared__ uint32_t carry_slot;  // the last candidate of the chunk before, INVALID_ID if it was not needed
     const uint32_t lt = (1u << lane) - 1u;
     for (uint32_t g = bk.idx; g < ng; g += bk.cnt) {
         const uint32_t s_first = g * GRPW;
@@ -591,7 +589,6 @@ DYN_KERNEL(__launch_bounds__(UT), k_group_union, (, bool force), (, force)) {
             io[tid] = make_float4(p.x, p.y, p.z, v.wid[s] != INVALID_ID ? 1.f : 0.f);
             v.wprune[s] = p;
         }
-        if (tid == 0) carry_slot = INVALID_ID;
         uint32_t* tl = v.tile_j + (size_t)g * v.cap_tile;
         const float4 c0 = v.gbb_c[g], h0 = v.gbb_h[g];
         uint32_t nt = 0;
@@ -625,7 +622,7 @@ DYN_KERNEL(__launch_bounds__(UT), k_group_union, (, bool force), (, force)) {
         }
         const uint32_t vm = __ballot_sync(0xffffffffu, io[lane].w != 0.f);  // the members
         uint32_t n_out[MPW] = {}, n_in[MPW] = {};
-        uint32_t base_cnt = 0, base_run = 0;
+        uint32_t base_cnt = 0;
         const uint32_t ncand = nt * WCL;
         for (uint32_t k0 = 0; k0 < ncand; k0 += UT) {
             const uint32_t k = k0 + tid;
@@ -652,13 +649,8 @@ DYN_KERNEL(__launch_bounds__(UT), k_group_union, (, bool force), (, force)) {
             const uint32_t mn = __ballot_sync(0xffffffffu, need);
             sh_out[tid] = mo;
             sh_in[tid] = mi;
-            sh_slot[tid] = need ? slot : INVALID_ID;
             if (lane == 0) wn[wid_] = __popc(mn);
             __syncthreads();
-            const uint32_t ps = tid ? sh_slot[tid - 1] : carry_slot;  // needed predecessor
-            const bool start = need && (ps == INVALID_ID || slot != ps + 1u);
-            const uint32_t ms = __ballot_sync(0xffffffffu, start);
-            if (lane == 0) wr[wid_] = __popc(ms);
             uint32_t loc = base_cnt + __popc(mn & lt), tn = 0;
 #pragma unroll
             for (int w = 0; w < NWP; ++w) {
@@ -669,16 +661,7 @@ DYN_KERNEL(__launch_bounds__(UT), k_group_union, (, bool force), (, force)) {
             sh_loc[tid] = fits ? (uint16_t)loc : (uint16_t)0xFFFFu;
             if (fits) v.grp_uslot[(size_t)g * v.cap_union + loc] = slot;
             __syncthreads();
-            uint32_t rid = base_run + __popc(ms & lt), tr = 0;
-#pragma unroll
-            for (int w = 0; w < NWP; ++w) {
-                if (w < wid_) rid += wr[w];
-                tr += wr[w];
-            }
-            if (start && rid < v.cap_run) v.grp_run[(size_t)g * v.cap_run + rid] = make_uint2(slot, loc);
             base_cnt += tn;
-            base_run += tr;
-            if (tid == 0) carry_slot = sh_slot[UT - 1];
             // the lists: members wid_ * MPW + q, 32 candidates at a time
             for (int c = 0; c < UT; c += 32) {
                 if (k0 + c >= ncand) break;
@@ -700,10 +683,8 @@ DYN_KERNEL(__launch_bounds__(UT), k_group_union, (, bool force), (, force)) {
         }
         if (tid == 0) {
             v.grp_nloc[g] = min(base_cnt, v.cap_union);
-            v.grp_nrun[g] = min(base_run, v.cap_run);
             if (base_cnt > v.cap_union) atomicMax(&v.sc->overflow, base_cnt);
             atomicMax(&v.sc->union_max, base_cnt);
-            if (base_run > v.cap_run) atomicMax(&v.sc->overflow, base_run);
         }
         if (lane == 0) {
 #pragma unroll
@@ -712,6 +693,25 @@ DYN_KERNEL(__launch_bounds__(UT), k_group_union, (, bool force), (, force)) {
                 v.wnb_n[s] = min(n_out[q], v.cap_nb);
                 v.winb_n[s] = min(n_in[q], v.cap_nb);
                 if (n_out[q] > v.cap_nb) atomicMax(&v.sc->overflow, n_out[q]);
+            }
+        }
+        if (v.ww_split > 1u) {
+            // where the parts of the union start in each pruned list
+            const uint32_t nloc = min(base_cnt, v.cap_union);
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < MPW; ++q) {
+                const uint32_t s = s_first + wid_ * MPW + q;
+                if ((uint32_t)lane < v.ww_split) {
+                    const uint16_t* lst = v.winb + (size_t)s * v.cap_nb;
+                    const uint32_t c = ww_cut(nloc, lane, v.ww_split);
+                    uint32_t l0 = 0, l1 = min(n_in[q], v.cap_nb);
+                    while (l0 < l1) {
+                        const uint32_t m = (l0 + l1) >> 1;
+                        if ((uint32_t)lst[m] < c) l0 = m + 1; else l1 = m;
+                    }
+                    v.winb_cut[(size_t)WW_SPLIT_MAX * s + lane] = (uint16_t)l0;
+                }
             }
         }
     }
@@ -749,6 +749,9 @@ DYN_KERNEL(__launch_bounds__(PRT), k_ww_prune, (, bool force), (, force)) {
         const uint32_t nloc = v.grp_nloc[g];
         const uint32_t s0 = g * GRPW + wp * MPW;
         uint32_t n[MPW], k0[MPW] = {}, cnt[MPW] = {}, nx[MPW];
+        // lane p counts the entries below the start of the union's part p
+        const uint32_t my_cut = (uint32_t)lane < v.ww_split ? ww_cut(nloc, lane, v.ww_split) : 0u;
+        uint32_t below[MPW] = {};
         float3 io[MPW];
 #pragma unroll
         for (int q = 0; q < MPW; ++q) {
@@ -783,6 +786,12 @@ DYN_KERNEL(__launch_bounds__(PRT), k_ww_prune, (, bool force), (, force)) {
                     const uint32_t mh = __ballot_sync(0xffffffffu, hit);
                     if (hit) out[cnt[q] + __popc(mh & lt)] = (uint16_t)idx;
                     cnt[q] += __popc(mh);
+                    for (uint32_t p = 1; p < v.ww_split; ++p) {
+                        const uint32_t cut = __shfl_sync(0xffffffffu, my_cut, p);
+                        const bool lower = hit & (idx < cut);
+                        const uint32_t c = __popc(__ballot_sync(0xffffffffu, lower));
+                        if ((uint32_t)lane == p) below[q] += c;
+                    }
                     k0[q] += adv;
                     if (adv < 32u) {
                         // the rest of these 32 belongs to the next chunk
@@ -799,6 +808,10 @@ DYN_KERNEL(__launch_bounds__(PRT), k_ww_prune, (, bool force), (, force)) {
 #pragma unroll
         for (int q = 0; q < MPW; ++q)
             if (lane == 0) v.winb_n[s0 + q] = cnt[q];
+#pragma unroll
+        for (int q = 0; q < MPW; ++q)
+            if (v.ww_split > 1u && (uint32_t)lane < v.ww_split)
+                v.winb_cut[(size_t)WW_SPLIT_MAX * (s0 + q) + lane] = (uint16_t)below[q];
         if (tid < GRPW) v.wprune[g * GRPW + tid] = v.wpos[4 * (g * GRPW + tid)];
     }
 }

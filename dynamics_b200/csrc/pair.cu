@@ -7,9 +7,9 @@
 // between charged sites, 1-2/1-3 exclusions, no intra-water pairs; 1-4 pairs
 // are excluded here and evaluated (scaled) by k_pair14.
 //
-// Work decomposition.  Water-water (full list, no atomics): one CTA per
-// 32-water i-group, j sites staged in shared memory, LPW lanes per i-water
-// over its compact molecule list (k_pair_ww_tile).  Atom-water and atom-atom
+// Work decomposition.  Water-water: one CTA per
+// 32-water i-group, j sites staged in shared memory, the group's molecule
+// lists dealt out over the threads (k_pair_ww_tile).  Atom-water and atom-atom
 // (half lists: every pair once): one warp per work item (an 8-body
 // i-cluster and up to ch_mix entries of its list); lane = (ii, jq) with
 // ii = lane & 7 and jq = lane >> 3 evaluates i-body ii against j-atoms jq and
@@ -23,6 +23,8 @@
 // the lanes of a j-body.  Integer sums do not depend on order, so the
 // result is deterministic.
 #include <algorithm>
+#include <cstring>
+#include <vector>
 
 #include "engine.cuh"
 
@@ -48,25 +50,25 @@ struct Acc3 {
 // r >= rc (src/cuda/cuda.cu:160-164).  On energy steps the energy
 // qqe erfc(alpha r) / r is added in float64.
 template <bool ENERGY>
-__device__ __forceinline__ void coul(float3 pi, float3 pj, float3 sh, float qq, double qqe, const SysView& v,
+__device__ __forceinline__ void coul(float3 pi, float3 pj, float3 sh, float qq, double qqe, const PairParams& P,
                                      float3& f, Acc3& a) {
     const float3 d = pi - (pj - sh);
     const float r2 = dot3(d, d);
     const float rinv = rsqrtf(r2);
-    const float t = fmaf(r2, v.two_over_rc2, -1.0f);
-    float g = v.poly_g[NPOLY_G - 1];
+    const float t = fmaf(r2, P.two_over_rc2, -1.0f);
+    float g = P.poly_g[NPOLY_G - 1];
 #pragma unroll
-    for (int k = NPOLY_G - 2; k >= 0; --k) g = fmaf(g, t, v.poly_g[k]);
+    for (int k = NPOLY_G - 2; k >= 0; --k) g = fmaf(g, t, P.poly_g[k]);
     float fs = qq * fmaf(rinv * rinv, rinv, g);
-    fs = r2 < v.rc2 ? fs : 0.0f;
+    fs = r2 < P.rc2 ? fs : 0.0f;
     f.x = fmaf(fs, d.x, f.x); f.y = fmaf(fs, d.y, f.y); f.z = fmaf(fs, d.z, f.z);
     a.w = fmaf(fs, r2, a.w);
-    if (ENERGY && r2 < v.rc2) {
+    if (ENERGY && r2 < P.rc2) {
         // erfc(alpha r) / r in float32 from the force's r^2 and 1/r, scaled by
         // the float64 charge product and summed in float64: per-pair errors
         // of a few ulp with no common sign
         const float re = r2 * rinv;
-        a.e_c += qqe * (double)(erfcf(v.alpha * re) * rinv);
+        a.e_c += qqe * (double)(erfcf(P.alpha * re) * rinv);
     }
 }
 
@@ -156,123 +158,105 @@ __device__ __forceinline__ void write_partials(const SysView& v, Blk bk, int reg
 }
 
 // ---------------------------------------------------------------------------
-// Staging for the water-water kernel (k_pair_ww_tile, below): a group's
-// union of j-waters, stored as runs of consecutive slots, is copied global
-// -> shared with one cp.async.bulk per run, completing on an mbarrier, with
-// bounded waits; the kernel then reads the j sites from shared memory
-// (4 x 16-byte loads per molecule pair).
+// Staging for the water-water kernel (k_pair_ww_tile, below): the sites of a
+// range of a group's union, 64 bytes per water, into shared memory with
+// asynchronous 16-byte copies.  Site k of union water u sits at 4 u + (k ^
+// swizzle(u)): lanes that read the same site of scattered waters then spread
+// over all eight 16-byte bank groups (unswizzled, a site falls into two of
+// them, and the four loads per molecule pair were 9-way conflicts on
+// average; bulk copies cannot write this order).
 // ---------------------------------------------------------------------------
-constexpr int WT = GRPW * LPW;  // threads per CTA
-constexpr uint32_t WAIT_LIMIT = 1u << 22;
+constexpr int WT = 256;  // threads per CTA
+constexpr int JS = 13;   // words per union water of the j sums
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait: gives up after WAIT_LIMIT polls and reports it
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned int* timeout_flag) {
-    for (uint32_t it = 0; it < WAIT_LIMIT; ++it)
-        if (mbar_try_wait(bar, parity)) return true;
-    atomicExch(timeout_flag, 1u);
-    return false;
-}
+__device__ __forceinline__ uint32_t tile_swizzle(uint32_t u) { return (u >> 1) & 3u; }
 
-// Issues the bulk copies that bring union entries [lo, hi) of group g (from
-// its runs of consecutive slots) into buf; one lane per run.  Called by one
-// whole warp; lane 0 arms the barrier with the byte count.
-__device__ __forceinline__ uint32_t stage_chunk(const SysView& v, uint32_t g, uint32_t lo, uint32_t hi,
-                                                float4* buf, uint64_t* bar, int lane, uint32_t* uslot = nullptr) {
-    const uint32_t nloc = v.grp_nloc[g], nrun = v.grp_nrun[g];
-    const uint2* runs = v.grp_run + (size_t)g * v.cap_run;
-    if (lane == 0) mbar_expect_tx(bar, (hi - lo) * (uint32_t)(4 * sizeof(float4)));
-    __syncwarp();
-    for (uint32_t t = lane; t < nrun; t += 32) {
-        const uint2 r = runs[t];
-        const uint32_t end = t + 1 < nrun ? runs[t + 1].y : nloc;
-        const uint32_t a = max(r.y, lo), e = min(end, hi);
-        if (a < e) {
-            bulk_g2s(buf + (size_t)(a - lo) * 4, v.wpos + (size_t)(r.x + (a - r.y)) * 4,
-                     (e - a) * (uint32_t)(4 * sizeof(float4)), bar);
-            if (uslot)
-                for (uint32_t u = a; u < e; ++u) uslot[u - lo] = r.x + (u - r.y);
-        }
+template <int T>
+__device__ __forceinline__ void stage_chunk(const SysView& v, uint32_t g, uint32_t lo, uint32_t n, float4* tile,
+                                            uint32_t* uslot, int tid) {
+    const uint32_t* slots = v.grp_uslot + (size_t)g * v.cap_union + lo;
+    for (uint32_t t = tid; t < 4 * n; t += T) {
+        const uint32_t u = t >> 2, k = t & 3u;
+        const uint32_t s = slots[u];
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(tile + 4 * u + (k ^ tile_swizzle(u))));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(v.wpos + 4 * (size_t)s + k) : "memory");
+        if (k == 0) uslot[u] = s;
     }
-    return hi - lo;
 }
 
-// Screened Coulomb of one site pair of a molecule pair, both sides: the
-// pair force fs d (d = pi - pj) is added to the i-site sum fi and to the
-// j-site sum gj (the j site receives -gj).
+// 1 / sqrt(x), the instruction behind rsqrtf; squared distances are never
+// subnormal, so the flushing form needs no scaling around it
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ void axpy3(float3& acc, float s, float3 d) {
+    acc.x = fmaf(s, d.x, acc.x); acc.y = fmaf(s, d.y, acc.y); acc.z = fmaf(s, d.z, acc.z);
+}
+
+// Screened Coulomb of one site pair of a molecule pair (coul above; nj is the
+// negated j position, moved to the image nearest the i-water): the pair
+// force fs d is added to the i-site sum fi and to gj (the j site receives
+// -gj).
 template <bool ENERGY>
-__device__ __forceinline__ void coul2(float3 pi, float3 pj, float qq, double qqe, const SysView& v, float3& fi,
+__device__ __forceinline__ void coul2(float3 pi, float3 nj, float qq, double qqe, const PairParams& P, float3& fi,
                                       float3& gj, Acc3& a) {
-    const float3 d = pi - pj;
+    const float3 d = pi + nj;
     const float r2 = dot3(d, d);
-    const float rinv = rsqrtf(r2);
-    const float t = fmaf(r2, v.two_over_rc2, -1.0f);
-    float g = v.poly_g[NPOLY_G - 1];
+    const float rinv = rsqrt_ftz(r2);
+    const float t = fmaf(r2, P.two_over_rc2, -1.0f);
+    float g = P.poly_g[NPOLY_G - 1];
 #pragma unroll
-    for (int k = NPOLY_G - 2; k >= 0; --k) g = fmaf(g, t, v.poly_g[k]);
+    for (int k = NPOLY_G - 2; k >= 0; --k) g = fmaf(g, t, P.poly_g[k]);
     float fs = qq * fmaf(rinv * rinv, rinv, g);
-    fs = r2 < v.rc2 ? fs : 0.0f;
-    fi.x = fmaf(fs, d.x, fi.x); fi.y = fmaf(fs, d.y, fi.y); fi.z = fmaf(fs, d.z, fi.z);
-    gj.x = fmaf(fs, d.x, gj.x); gj.y = fmaf(fs, d.y, gj.y); gj.z = fmaf(fs, d.z, gj.z);
+    fs = r2 < P.rc2 ? fs : 0.0f;
+    axpy3(fi, fs, d);
+    axpy3(gj, fs, d);
     a.w = fmaf(fs, r2, a.w);
-    if (ENERGY && r2 < v.rc2) {
-        const float re = r2 * rinv;
-        a.e_c += qqe * (double)(erfcf(v.alpha * re) * rinv);
-    }
+    if (ENERGY && r2 < P.rc2) a.e_c += qqe * (double)(erfcf(P.alpha * (r2 * rinv)) * rinv);
 }
 
-// j-side forces of union water u are added to the CTA's int32 sums; a
-// molecule pair with a component too large for them (|f| >= JFIX_MAX: 32
-// such contributions stay below 2^15 kcal/mol/A, the int32 range at
-// 2^-16) goes to the slot's int64 overflow sums instead.  Which path a pair
-// takes depends only on its values, and both are integer sums, so the
-// result stays deterministic.
+// j-side forces of a union water are added to the CTA's int32 sums.  A
+// component too large for them (|f| >= JFIX_MAX: 32 such contributions stay
+// below 2^15 kcal/mol/A, the int32 range at 2^-16) takes its whole site out
+// of the sums (sites with one are flagged), and the molecule pair is
+// evaluated again by jforce_big, which adds the flagged sites' forces to the
+// slot's int64 sums.  Which way a site goes depends only on its values, and
+// both are integer sums, so the result stays deterministic.
 constexpr float JFIX_SCALE = (float)(1 << WW_JFIX_SHIFT);
 constexpr float JFIX_MAX = 1000.0f;
 
-__device__ __noinline__ void jforce_big(const SysView& v, uint32_t g, uint32_t u, int c, float f) {
-    const uint32_t slot = v.grp_uslot[(size_t)g * v.cap_union + u];
-    fix_atomic_add(v.wforce + (size_t)slot * 12 + c, fix_from_float(f));
+// The force -g on one site into its three sums; true if it did not fit.
+__device__ __forceinline__ bool jforce_add3(int* p, float3 g) {
+    const bool big = fmaxf(fmaxf(fabsf(g.x), fabsf(g.y)), fabsf(g.z)) >= JFIX_MAX;
+    const float sc = big ? 0.0f : -JFIX_SCALE;
+    atomicAdd(p + 0, __float2int_rn(g.x * sc));
+    atomicAdd(p + 1, __float2int_rn(g.y * sc));
+    atomicAdd(p + 2, __float2int_rn(g.z * sc));
+    return big;
 }
 
-// The 12 j-side components of one molecule pair (the forces on the j
-// water's O, H0, H1, M); one range check for all of them.
-__device__ __forceinline__ void jforce_add12(const SysView& v, int* jacc, uint32_t cs, uint32_t g, uint32_t u,
-                                             uint32_t ul, const float (&f)[12]) {
-    float m = 0.f;
-#pragma unroll
-    for (int c = 0; c < 12; ++c) m = fmaxf(m, fabsf(f[c]));
-    if (m < JFIX_MAX) {
-#pragma unroll
-        for (int c = 0; c < 12; ++c) atomicAdd(jacc + (size_t)c * cs + ul, __float2int_rn(f[c] * JFIX_SCALE));
-    } else {
-        for (int c = 0; c < 12; ++c) jforce_big(v, g, u, c, f[c]);
+// The flagged sites (bit k: site k) of the j water in slot, whose negated
+// sites nj are at the image nearest the i-water pi.
+__device__ __noinline__ void jforce_big(const SysView& v, uint32_t slot, uint32_t sites, const float4* pi,
+                                        const float4* pj, uint32_t sw, float3 n) {
+    const BoxDev b = *v.box;
+    const float q[3] = {OPC_Q_H, OPC_Q_H, OPC_Q_EP};
+    for (int k = 0; k < 4; ++k) {
+        if (!((sites >> k) & 1u)) continue;
+        const float4 p0 = pj[k ^ sw];
+        const float3 j = f3(-fmaf(n.x, b.ext[0], -p0.x), -fmaf(n.y, b.ext[1], -p0.y), -fmaf(n.z, b.ext[2], -p0.z));
+        float3 f = f3(0.f, 0.f, 0.f);
+        Acc3 a{0.0, 0.0, 0.f, 0.0};
+        if (k == 0) lj<false>(xyz(pi[0]), j, f3(0.f, 0.f, 0.f), OPC_O_SIGMA * OPC_O_SIGMA, OPC_O_EPS, v.pp.ljc2, 1.0f, f, a);
+        for (int i = 1; i < 4 && k; ++i)
+            coul<false>(xyz(pi[i]), j, f3(0.f, 0.f, 0.f), q[i - 1] * q[k - 1], 0.0, v.pp, f, a);
+        long long* p = v.wforce + (size_t)slot * 12 + 3 * k;
+        fix_atomic_add(p + 0, fix_from_float(-f.x));
+        fix_atomic_add(p + 1, fix_from_float(-f.y));
+        fix_atomic_add(p + 2, fix_from_float(-f.z));
     }
 }
 
@@ -291,130 +275,109 @@ __device__ __forceinline__ void write_partials_warp(const SysView& v, Blk bk, in
 }
 
 // ---------------------------------------------------------------------------
-// water(i) - water(j), tile form, half lists.  One CTA per 32-water
-// i-group.  The waters the group's lists reach (its union, stored as runs
-// of consecutive slots) are copied global -> shared with one cp.async.bulk
-// per run, completing on an mbarrier, union_chunk waters at a time (one
-// chunk for most groups; sized so that three CTAs fit on an SM, with 80
-// registers per thread; the batch form, which reads its SysView from global
-// memory, spills at 80 and runs two CTAs per SM instead).  The lists hold
-// every water pair once (in the list of the lower slot), so
-// their lengths vary several-fold across a group; the chunk's entries of
-// all 32 lists are therefore dealt out as one sequence, an equal
-// contiguous share per thread, whatever list they come from.  A thread
-// keeps the i-water's forces in registers while its share stays in one
-// list and adds them to the water forces (int64 reductions) when it moves
-// to the next list.  All 10 site pairs of a molecule pair use one
-// min-image shift.  The j-side forces are summed per union water in shared
-// memory (int32 fixed point, 12 components, component-major with a stride
-// of chunk + 1 words, so that both the threads' adds and the flush's reads
-// spread over the banks), then added to the union waters' forces with one
-// coalesced run of int64 reductions per chunk (the union's slots are noted
-// in shared memory while the copies are issued).  The shares depend only on
-// the lists and the chunk size, and every sum across threads is an integer
-// sum: the forces are the same bits run to run.  The list lengths of a group
-// whose union fits one chunk (almost every group) are read while its copies
-// are in flight; larger unions find each chunk's entries by binary search.
-// A system with fewer groups than the GPU has SMs gives each group ww_split
-// CTAs, each staging the union and taking an equal slice of the entries.
+// water(i) - water(j), tile form, half lists.  A unit of work is a 32-water
+// i-group and one of ww_split equal ranges of its union (the waters its
+// lists reach); a CTA per unit copies the range's sites to shared memory, at
+// most union_chunk waters at a time (one chunk for most
+// units).  The lists hold every water pair once (in the list of the lower
+// slot), so their lengths vary several-fold across a group; the chunk's
+// entries of all 32 lists are therefore dealt out as one sequence, an equal
+// contiguous share per thread, whatever list they come from.  A thread keeps
+// the i-water's forces in registers while its share stays in one list and
+// adds them to the water forces (int64 reductions) when it moves to the
+// next.  All 10 site pairs of a molecule pair use one min-image shift.  The
+// j sites are taken one after another, so that only one site's j force is
+// held at a time: it goes to int32 fixed-point sums in shared memory (12
+// components, 13 words apart per water, so that the threads' adds spread over
+// the banks and take fixed offsets), which are added to the union waters'
+// forces with one coalesced run of int64 reductions per chunk.  The shares
+// depend only on the lists, the split and the chunk size, and every sum
+// across threads is an integer sum: the forces are the same bits run to run.
+//
+// 24,000 waters in 98 A: 2.2 M list entries.  What it waits for is the
+// latency of the shared-memory gathers, the barriers around each unit and the
+// last wave of units (3 CTAs per SM; the batch form, which holds the view's
+// pointers in registers, spills there and runs 2: 64 systems 1244 us a step
+// against 1312).  84 -> 71 us (80,000 waters 217 -> 185, 8,000 waters 57 ->
+// 39, 512 waters 22 -> 17) by the swizzled tile (the gathers were 9-way bank
+// conflicts, 63 % of the shared-memory wavefronts), j sums at fixed offsets,
+// one check for large forces per molecule pair instead of a branch per site,
+// image shifts by fused multiply-adds, and parts that stage, zero and flush
+// their own range of the union only (a part used to handle all of it).  Two
+// entries at a time in packed float32 registers ran 38 M instead of 46 M
+// instructions but no faster: a third of its instructions duplicated
+// coefficients into register pairs, at 2 CTAs per SM.
 // ---------------------------------------------------------------------------
-DYN_KERNEL_T2((bool ENERGY), (ENERGY), __launch_bounds__(WT, 3), __launch_bounds__(WT, 2), k_pair_ww_tile, (), ()) {
+DYN_KERNEL_T2((bool ENERGY), (ENERGY), __launch_bounds__(WT, 3), __launch_bounds__(WT, 2), k_pair_ww_tile, (, const PairParams P), (, P)) {
     extern __shared__ __align__(128) float4 tile[];  // union_chunk waters x 4 float4, then the j sums
-    __shared__ __align__(8) uint64_t bar;
     __shared__ float4 ipos[GRPW * 4];   // the group's i-water sites
     __shared__ uint32_t woff[GRPW + 1]; // first share position of each list's chunk entries
     __shared__ uint32_t wbeg[GRPW];     // each list's first entry in the chunk
     __shared__ uint32_t wend[GRPW];     // ... and one past its last
-    __shared__ uint32_t wlen[GRPW];     // list lengths
     const int tid = threadIdx.x;
     const uint32_t nwc = v.sc->n_wclus;
     const uint32_t ng = (nwc + GRPW / WCL - 1) / (GRPW / WCL);
-    const uint32_t nslots = nwc * WCL;
     const uint32_t chunk = v.union_chunk;
-    const uint32_t cs = chunk + 1;  // component stride of the j sums
-    int* jacc = reinterpret_cast<int*>(tile + 4 * (size_t)chunk);  // [12][chunk + 1]
-    uint32_t* uslot = reinterpret_cast<uint32_t*>(jacc + 12 * (size_t)cs);  // [chunk] union entry -> slot
+    int* jacc = reinterpret_cast<int*>(tile + 4 * (size_t)chunk);            // [chunk][JS], 12 used
+    uint32_t* uslot = reinterpret_cast<uint32_t*>(jacc + JS * (size_t)chunk);  // [chunk] union entry -> slot
     const BoxDev b = *v.box;
-    const float ljc2 = v.ljc2;
-    const float sig2 = OPC_O_SIGMA * OPC_O_SIGMA;
-    const float qhh = OPC_Q_H * OPC_Q_H, qhm = OPC_Q_H * OPC_Q_EP, qmm = OPC_Q_EP * OPC_Q_EP;
+    constexpr float qhh = OPC_Q_H * OPC_Q_H, qhm = OPC_Q_H * OPC_Q_EP, qmm = OPC_Q_EP * OPC_Q_EP;
     const double ehh = (double)OPC_Q_H * (double)OPC_Q_H, ehm = (double)OPC_Q_H * (double)OPC_Q_EP,
                  emm = (double)OPC_Q_EP * (double)OPC_Q_EP;
-    if (tid == 0) mbar_init(&bar, 1);
-    // the j sums start at zero; each chunk's flush zeroes what it read
-    for (uint32_t t = tid; t < 12 * cs; t += WT) jacc[t] = 0;
-    __syncthreads();
-    uint32_t parity = 0;
     Acc3 a{0.0, 0.0, 0.f, 0.0};
-    bool alive = true;
-    // inclusive scan of a count over the 32 lanes of a warp
-    auto scan32 = [](uint32_t x, int l) {
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (l >= o) x += y;
-        }
-        return x;
-    };
     const uint32_t split = v.ww_split;
-    for (uint32_t q = bk.idx; q < ng * split && alive; q += bk.cnt) {
+    for (uint32_t q = bk.idx; q < ng * split; q += bk.cnt) {
         const uint32_t g = q / split, part = q - g * split;
         const uint32_t nloc = v.grp_nloc[g];
-        if (tid < GRPW * 4) {
-            const uint32_t s = g * GRPW + tid / 4;
-            ipos[tid] = s < nslots ? v.wpos[(size_t)4 * g * GRPW + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        const bool single = nloc <= chunk;
+        const uint32_t plo = ww_cut(nloc, part, split), phi = ww_cut(nloc, part + 1, split);
+        if (tid < GRPW * 4) ipos[tid] = v.wpos[(size_t)4 * g * GRPW + tid];  // nw_cap holds whole groups
+        uint32_t wlen = 0;
         if (tid >= 32 && tid < 32 + GRPW) {
+            // this part's entries of list w: [wend, wlen)
             const int w = tid - 32;
             const uint32_t s = g * GRPW + w;
-            const uint32_t n = s < nslots ? v.winb_n[s] : 0u;
-            wlen[w] = n;
-            wend[w] = 0u;
-            if (single) {
-                // one chunk: every entry of every list
-                const uint32_t x = scan32(n, w);
-                wbeg[w] = 0u;
-                woff[w + 1] = x;
-                if (w == 0) woff[0] = 0u;
+            wlen = v.winb_n[s];
+            uint32_t b0 = 0;
+            if (split > 1) {
+                const uint16_t* cut = v.winb_cut + (size_t)WW_SPLIT_MAX * s;
+                if (part) b0 = cut[part];
+                if (part + 1 < split) wlen = cut[part + 1];
             }
+            wend[w] = b0;
         }
-        for (uint32_t lo = 0; lo < nloc; lo += chunk) {
-            const uint32_t hi = min(nloc, lo + chunk);
-            if (tid < 32) stage_chunk(v, g, lo, hi, tile, &bar, tid, uslot);
-            __syncthreads();  // the lengths and wend of the previous chunk are visible
-            if (!single && tid >= 32 && tid < 32 + GRPW) {
+        for (uint32_t lo = plo; lo < phi; lo += chunk) {
+            const uint32_t hi = min(phi, lo + chunk), nu = hi - lo;
+            stage_chunk<WT>(v, g, lo, nu, tile, uslot, tid);
+            if (tid >= 32 && tid < 32 + GRPW) {
                 // the list entries of this chunk: from where the previous
                 // chunk stopped to the first union index >= hi (lists ascend)
                 const int w = tid - 32;
-                const uint16_t* lst = v.winb + (size_t)(g * GRPW + w) * v.cap_nb;
                 const uint32_t b0 = wend[w];
-                uint32_t l0 = b0, l1 = wlen[w];
+                uint32_t l0 = b0, l1 = wlen;
+                if (hi == phi) l0 = l1;
+                const uint16_t* lst = v.winb + (size_t)(g * GRPW + w) * v.cap_nb;
                 while (l0 < l1) {
                     const uint32_t m = (l0 + l1) >> 1;
                     if ((uint32_t)lst[m] < hi) l0 = m + 1; else l1 = m;
                 }
-                const uint32_t x = scan32(l0 - b0, w);
+                uint32_t x = l0 - b0;  // inclusive scan over the lists
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (w >= o) x += y;
+                }
                 wbeg[w] = b0;
                 woff[w + 1] = x;
                 if (w == 0) woff[0] = 0u;
                 wend[w] = l0;
             }
-            const bool ok = mbar_wait(&bar, parity, &v.sc->timeout);
-            if (!__syncthreads_and(ok)) {
-                // give the copies in flight one more bounded chance, then stop
-                if (!ok) mbar_wait(&bar, parity, &v.sc->timeout);
-                alive = false;
-                break;
-            }
-            parity ^= 1u;
-            // this CTA's slice of the chunk's entries, and this thread's
-            // share [e0, e1) of the slice
+            for (uint32_t t = tid; t < JS * nu; t += WT) jacc[t] = 0;  // the j sums start at zero
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            // this thread's share of the entries
             const uint32_t total = woff[GRPW];
-            const uint32_t s0 = (uint32_t)(((uint64_t)part * total) / split);
-            const uint32_t slen = (uint32_t)(((uint64_t)(part + 1) * total) / split) - s0;
-            const uint32_t e0 = s0 + (uint32_t)(((uint64_t)tid * slen) / WT);
-            const uint32_t e1 = s0 + (uint32_t)(((uint64_t)(tid + 1) * slen) / WT);
+            const uint32_t e0 = (uint32_t)(((uint64_t)tid * total) / WT);
+            const uint32_t e1 = (uint32_t)(((uint64_t)(tid + 1) * total) / WT);
             int w = 0;
             while (w < GRPW - 1 && woff[w + 1] <= e0) ++w;
             float3 iO = f3(0, 0, 0), iH0 = iO, iH1 = iO, iM = iO;
@@ -446,52 +409,54 @@ DYN_KERNEL_T2((bool ENERGY), (ENERGY), __launch_bounds__(WT, 3), __launch_bounds
                     enter(wn);
                     idx_next = (uint32_t)lst[e];
                 }
-                const uint32_t idx = idx_next;
+                const uint32_t u = idx_next - lo;
                 if (e + 1 < e1 && e + 1 < wstop) idx_next = (uint32_t)lst[e + 1];
-                const float4* jw = tile + 4 * (idx - lo);
-                const float3 jO = xyz(jw[0]);
-                const float3 sh = shift_of(iO - jO, b);
-                // the j sites moved by the shift once, then zero shift
-                const float3 z0 = f3(0.f, 0.f, 0.f);
-                const float3 sO = jO - sh, sH0 = xyz(jw[1]) - sh, sH1 = xyz(jw[2]) - sh, sM = xyz(jw[3]) - sh;
-                float3 gO = z0, gH0 = z0, gH1 = z0, gM = z0;
+                const float4* jw = tile + 4 * u;
+                const uint32_t sw = tile_swizzle(u);
+                int* jf = jacc + JS * u;
+                // negated j sites at the image nearest the i-water
+                const float3 jO = xyz(jw[sw]);
+                const float3 n = f3(-nearest_int(iO.x - jO.x, b.inv_ext[0]), -nearest_int(iO.y - jO.y, b.inv_ext[1]),
+                                    -nearest_int(iO.z - jO.z, b.inv_ext[2]));
+                auto image = [&](float3 p) {
+                    return f3(fmaf(n.x, b.ext[0], -p.x), fmaf(n.y, b.ext[1], -p.y), fmaf(n.z, b.ext[2], -p.z));
+                };
+                uint32_t big = 0;  // sites whose force does not fit the int32 sums
                 {
-                    float3 t = z0;
-                    lj<ENERGY>(iO, sO, z0, sig2, OPC_O_EPS, ljc2, 1.0f, t, a);
+                    const float3 nj = image(jO);
+                    float3 t = f3(0.f, 0.f, 0.f);
+                    lj<ENERGY>(iO, f3(-nj.x, -nj.y, -nj.z), f3(0.f, 0.f, 0.f), OPC_O_SIGMA * OPC_O_SIGMA, OPC_O_EPS,
+                               P.ljc2, 1.0f, t, a);
                     fO = fO + t;
-                    gO = t;
+                    if (jforce_add3(jf, t)) big |= 1u;
                 }
-                coul2<ENERGY>(iH0, sH0, qhh, ehh, v, fH0, gH0, a);
-                coul2<ENERGY>(iH0, sH1, qhh, ehh, v, fH0, gH1, a);
-                coul2<ENERGY>(iH0, sM, qhm, ehm, v, fH0, gM, a);
-                coul2<ENERGY>(iH1, sH0, qhh, ehh, v, fH1, gH0, a);
-                coul2<ENERGY>(iH1, sH1, qhh, ehh, v, fH1, gH1, a);
-                coul2<ENERGY>(iH1, sM, qhm, ehm, v, fH1, gM, a);
-                coul2<ENERGY>(iM, sH0, qhm, ehm, v, fM, gH0, a);
-                coul2<ENERGY>(iM, sH1, qhm, ehm, v, fM, gH1, a);
-                coul2<ENERGY>(iM, sM, qmm, emm, v, fM, gM, a);
+#pragma unroll
+                for (int k = 1; k < 4; ++k) {
+                    const float3 nj = image(xyz(jw[k ^ sw]));
+                    float3 gj = f3(0.f, 0.f, 0.f);
+                    coul2<ENERGY>(iH0, nj, k == 3 ? qhm : qhh, k == 3 ? ehm : ehh, P, fH0, gj, a);
+                    coul2<ENERGY>(iH1, nj, k == 3 ? qhm : qhh, k == 3 ? ehm : ehh, P, fH1, gj, a);
+                    coul2<ENERGY>(iM, nj, k == 3 ? qmm : qhm, k == 3 ? emm : ehm, P, fM, gj, a);
+                    if (jforce_add3(jf + 3 * k, gj)) big |= 1u << k;
+                }
+                if (big) jforce_big(v, uslot[u], big, ipos + 4 * w, jw, sw, n);
                 a.flush_w();
-                // the j waters receive the opposite forces (sites O, H0, H1, M)
-                const float jf[12] = {-gO.x, -gO.y, -gO.z, -gH0.x, -gH0.y, -gH0.z,
-                                      -gH1.x, -gH1.y, -gH1.z, -gM.x, -gM.y, -gM.z};
-                jforce_add12(v, jacc, cs, g, idx, idx - lo, jf);
             }
             if (e0 < e1) leave();
             __syncthreads();  // every j sum of the chunk is in
             // the chunk's sums -> the union waters' forces (2^-16 -> 2^-32
             // fixed point); consecutive union entries of a run are
             // consecutive slots, so the reductions are coalesced
-            for (uint32_t t = tid; t < 12 * (hi - lo); t += WT) {
+            for (uint32_t t = tid; t < 12 * nu; t += WT) {
                 const uint32_t u = t / 12, c = t - 12 * u;
-                const int val = jacc[c * cs + u];
-                if (val != 0) {
-                    jacc[c * cs + u] = 0;
+                const int val = jacc[JS * u + c];
+                if (val != 0)
                     fix_atomic_add(v.wforce + 12 * (size_t)uslot[u] + c,
                                    (long long)val * (1ll << (32 - WW_JFIX_SHIFT)));
-                }
             }
-            __syncthreads();  // the tile and the sums are refilled by the next chunk or group
+            __syncthreads();  // the tile and the sums are refilled by the next chunk or unit
         }
+        __syncthreads();  // the i-water sites are refilled by the next unit
     }
     write_partials<ENERGY>(v, bk, REG_WW, ENERGY ? a.e_lj : 0.0, ENERGY ? a.e_c : 0.0, a.wd);
 }
@@ -536,14 +501,14 @@ __device__ __forceinline__ JAtoms load_jatoms(const SysView& v, uint32_t cj, int
 // forces) are reduce-scattered over the 8 water lanes of a j-group and added
 // with integer atomics (24 per entry).
 // ---------------------------------------------------------------------------
-DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT, 4), k_pair_ws, (), ()) {
+DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT, 4), k_pair_ws, (, const PairParams P), (, P)) {
     const int lane = threadIdx.x & 31;
     const int ii = lane & 7, jq = lane >> 3;
     const uint32_t nwarps = (bk.cnt * blockDim.x) >> 5;
     const uint32_t nit = v.sc->n_ws_items;
     const uint32_t first_single = v.sc->a_sparse_base / ACL;  // first single-atom cluster
     const BoxDev b = *v.box;
-    const float ljc2 = v.ljc2;
+    const float ljc2 = P.ljc2;
     double el = 0.0, ec = 0.0, ew = 0.0, dh = 0.0;
     for (uint32_t it = ((bk.idx * blockDim.x + threadIdx.x) >> 5); it < nit; it += nwarps) {
         const uint2 item = v.ws_item[it];
@@ -576,20 +541,24 @@ DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT, 4),
             const JAtoms cur = nx;
             k += advance(k);
             if (k < n) nx = load_at(k);
-            // the cluster boxes met within r_ws; skip the entry when no lane's
-            // water O lies within cutoff + O-H reach of its atoms
+            // the cluster boxes met within r_ws; skip the half (atoms 0-3 or
+            // 4-7) of the entry where no lane's water O lies within cutoff +
+            // O-H reach of an atom
+            bool near0, near1;
             {
                 const float r2 = v.r_ws_skip2;
-                bool near = false;
+                bool n0 = false, n1 = false;
                 if (vi && cur.a0 != INVALID_ID) {
-                    const float3 d = min_image_rint(iO - xyz(cur.p0), b);
-                    near = dot3(d, d) < r2;
+                    const float3 d = min_image_fast(iO - xyz(cur.p0), b);
+                    n0 = dot3(d, d) < r2;
                 }
                 if (vi && cur.a1 != INVALID_ID) {
-                    const float3 d = min_image_rint(iO - xyz(cur.p1), b);
-                    near = near || dot3(d, d) < r2;
+                    const float3 d = min_image_fast(iO - xyz(cur.p1), b);
+                    n1 = dot3(d, d) < r2;
                 }
-                if (!__any_sync(0xffffffffu, near)) continue;
+                near0 = __any_sync(0xffffffffu, n0);
+                near1 = __any_sync(0xffffffffu, n1);
+                if (!near0 && !near1) continue;
             }
             float jf[8];
 #pragma unroll
@@ -598,7 +567,7 @@ DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT, 4),
                 const float2 lj_j = h ? cur.l1 : cur.l0;
                 const uint32_t aj = h ? cur.a1 : cur.a0;
                 float3 fo = f3(0, 0, 0), f0 = fo, f1 = fo, fm = fo;
-                if (vi && aj != INVALID_ID) {
+                if ((h ? near1 : near0) && vi && aj != INVALID_ID) {
                     const float3 jp = xyz(pj);
                     // the atom moved by the shift once, then zero shift
                     const float3 js = jp - shift_of(iO - jp, b), z0 = f3(0.f, 0.f, 0.f);
@@ -609,18 +578,18 @@ DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT, 4),
                         // a water and an atom of the alchemical molecule
                         lj_soft<ENERGY>(iO, js, z0, sg, ep, ljc2, v.alch_ll, v.alch_dll, fo, a, dh);
                         Acc3 t{0.0, 0.0, 0.f, 0.0};
-                        coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, v, f0, t);
-                        coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, v, f1, t);
-                        coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, v, fm, t);
+                        coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f0, t);
+                        coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f1, t);
+                        coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, P, fm, t);
                         const float cs = v.alch_cs;
                         f0 = f0 * cs; f1 = f1 * cs; fm = fm * cs;
                         a.w = fmaf(cs, t.w, a.w);
                         if (ENERGY) { a.e_c += (double)cs * t.e_c; dh += (double)v.alch_dcs * t.e_c; }
                     } else {
                         lj<ENERGY>(iO, js, z0, sg * sg, ep, ljc2, 1.0f, fo, a);
-                        coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, v, f0, a);
-                        coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, v, f1, a);
-                        coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, v, fm, a);
+                        coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f0, a);
+                        coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f1, a);
+                        coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, P, fm, a);
                     }
                 }
                 fO = fO + fo; fH0 = fH0 + f0; fH1 = fH1 + f1; fM = fM + fm;
@@ -656,13 +625,13 @@ DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT, 4),
 // interaction mask from the list build holds jj > ii on the diagonal and
 // drops exclusions); work items, prefetch and j-side atomics as above.
 // ---------------------------------------------------------------------------
-DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT), k_pair_ss, (), ()) {
+DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT), k_pair_ss, (, const PairParams P), (, P)) {
     const int lane = threadIdx.x & 31;
     const int ii = lane & 7, jq = lane >> 3;
     const uint32_t nwarps = (bk.cnt * blockDim.x) >> 5;
     const uint32_t nit = v.sc->n_ss_items;
     const BoxDev b = *v.box;
-    const float ljc2 = v.ljc2;
+    const float ljc2 = P.ljc2;
     double el = 0.0, ec = 0.0, ew = 0.0, dh = 0.0;
     for (uint32_t it = ((bk.idx * blockDim.x + threadIdx.x) >> 5); it < nit; it += nwarps) {
         const uint2 item = v.ss_item[it];
@@ -699,14 +668,14 @@ DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT), k_
                                         fp, a, dh);
                         Acc3 t{0.0, 0.0, 0.f, 0.0};
                         float3 fc = f3(0.f, 0.f, 0.f);
-                        coul<ENERGY>(xyz(pi), xyz(pj), s, pi.w * pj.w, (double)pi.w * (double)pj.w, v, fc, t);
+                        coul<ENERGY>(xyz(pi), xyz(pj), s, pi.w * pj.w, (double)pi.w * (double)pj.w, P, fc, t);
                         const float cs = v.alch_cs;
                         fp = fp + fc * cs;
                         a.w = fmaf(cs, t.w, a.w);
                         if (ENERGY) { a.e_c += (double)cs * t.e_c; dh += (double)v.alch_dcs * t.e_c; }
                     } else {
                         lj<ENERGY>(xyz(pi), xyz(pj), s, sg * sg, sqrtf(lji.y * ljj.y), ljc2, 1.0f, fp, a);
-                        coul<ENERGY>(xyz(pi), xyz(pj), s, pi.w * pj.w, (double)pi.w * (double)pj.w, v, fp, a);
+                        coul<ENERGY>(xyz(pi), xyz(pj), s, pi.w * pj.w, (double)pi.w * (double)pj.w, P, fp, a);
                     }
                 }
                 f = f + fp;
@@ -733,7 +702,7 @@ DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT), k_
 // ---------------------------------------------------------------------------
 // 1-4 pairs: LJ x0.5, Coulomb x1/1.2 (src/non_bonded.rs:55-56,1014-1042)
 // ---------------------------------------------------------------------------
-DYN_KERNEL_T((bool ENERGY), (ENERGY), , k_pair14, (), ()) {
+DYN_KERNEL_T((bool ENERGY), (ENERGY), , k_pair14, (, const PairParams P), (, P)) {
     const BoxDev b = *v.box;
     double e_acc = 0.0, w_acc = 0.0;
     for (uint32_t k = bk.idx * blockDim.x + threadIdx.x; k < v.n14; k += bk.cnt * blockDim.x) {
@@ -743,10 +712,10 @@ DYN_KERNEL_T((bool ENERGY), (ENERGY), , k_pair14, (), ()) {
         const float3 sh = shift_of(xyz(pa) - xyz(pb), b);
         float3 f = f3(0, 0, 0);
         Acc3 a{0.0, 0.0, 0.f, 0.0};
-        lj<ENERGY>(xyz(pa), xyz(pb), sh, par.x * par.x, par.y, v.ljc2, 0.5f, f, a);
+        lj<ENERGY>(xyz(pa), xyz(pb), sh, par.x * par.x, par.y, P.ljc2, 0.5f, f, a);
         float3 fc = f3(0, 0, 0);
         Acc3 ac{0.0, 0.0, 0.f, 0.0};
-        coul<ENERGY>(xyz(pa), xyz(pb), sh, par.z, (double)pa.w * (double)pb.w, v, fc, ac);
+        coul<ENERGY>(xyz(pa), xyz(pb), sh, par.z, (double)pa.w * (double)pb.w, P, fc, ac);
         const float s = 0.833333333f;
         f = f + fc * s;
         add_fix3(v.aforce + 3 * (size_t)p.x, f);
@@ -779,10 +748,8 @@ int ww_tile_blocks(const SysView& v) {
     return (int)(n < v.max_blocks ? n : v.max_blocks);
 }
 
-// per union water: 4 float4 positions, 12 int32 j sums (+ the stride pad) and its slot
-size_t ww_tile_smem(const SysView& v) {
-    return (size_t)v.union_chunk * (4 * sizeof(float4) + 13 * sizeof(int)) + 12 * sizeof(int);
-}
+// per union water: 4 float4 positions, the j sums and its slot
+size_t ww_tile_smem(const SysView& v) { return (size_t)v.union_chunk * WW_CHUNK_BYTES; }
 
 // The limit is a property of the kernel, shared by every system in the
 // process, so it is raised to the device maximum once rather than set to one
@@ -819,13 +786,32 @@ inline bool any_alch(const Target& t) {
     return t.any([](const SysView& v) { return v.alch_on != 0u; });
 }
 
+// The pair kernels take the cutoffs and the force polynomial by value, so
+// that they read them as constants also where their SysView lies in global
+// memory (a batch): one launch for every distinct set among the systems, which
+// is one unless a batch's members differ in cutoff or alpha.
+template <typename KP, typename KB, typename G>
+void launch_pair_kernel(const Target& t, KP kp, KB kb, G grid, int threads, size_t smem) {
+    std::vector<PairParams> sets;
+    auto same = [](const PairParams& a, const PairParams& b) { return std::memcmp(&a, &b, sizeof(PairParams)) == 0; };
+    if (t.v) sets.push_back(t.v->pp);
+    else
+        for (uint32_t i = 0; i < batch_size(t.b); ++i) {
+            const PairParams& p = batch_view(t.b, i).pp;
+            if (std::none_of(sets.begin(), sets.end(), [&](const PairParams& q) { return same(p, q); }))
+                sets.push_back(p);
+        }
+    for (const PairParams& p : sets)
+        t.launch(kp, kb, [&](const SysView& v) { return same(v.pp, p) ? grid(v) : 0; }, threads, smem, p);
+}
+
 void launch_pairs_atoms(const Target& t, bool energy) {
     auto ss = [](const SysView& v) { return v.na ? pair_blocks_ss(v) : 0; };
     const bool al = any_alch(t);
-    if (energy && al) t.launch(k_pair_ss<true, true>, k_pair_ss_batch<true, true>, ss, PT, 0);
-    else if (energy) t.launch(k_pair_ss<true, false>, k_pair_ss_batch<true, false>, ss, PT, 0);
-    else if (al) t.launch(k_pair_ss<false, true>, k_pair_ss_batch<false, true>, ss, PT, 0);
-    else t.launch(k_pair_ss<false, false>, k_pair_ss_batch<false, false>, ss, PT, 0);
+    if (energy && al) launch_pair_kernel(t, k_pair_ss<true, true>, k_pair_ss_batch<true, true>, ss, PT, 0);
+    else if (energy) launch_pair_kernel(t, k_pair_ss<true, false>, k_pair_ss_batch<true, false>, ss, PT, 0);
+    else if (al) launch_pair_kernel(t, k_pair_ss<false, true>, k_pair_ss_batch<false, true>, ss, PT, 0);
+    else launch_pair_kernel(t, k_pair_ss<false, false>, k_pair_ss_batch<false, false>, ss, PT, 0);
 }
 
 void launch_pairs_ww(const Target& t, bool energy) {
@@ -834,10 +820,10 @@ void launch_pairs_ww(const Target& t, bool energy) {
     // DYN_FLAG_FULL_ENERGY (the reference leaves it out,
     // src/non_bonded.rs:335-342), so other energy steps skip it
     auto eww = [energy](const SysView& v) { return energy && (v.flags & DYN_FLAG_FULL_ENERGY); };
-    t.launch(k_pair_ww_tile<true>, k_pair_ww_tile_batch<true>,
-             [&](const SysView& v) { return v.nw && eww(v) ? ww_tile_blocks(v) : 0; }, WT, sm);
-    t.launch(k_pair_ww_tile<false>, k_pair_ww_tile_batch<false>,
-             [&](const SysView& v) { return v.nw && !eww(v) ? ww_tile_blocks(v) : 0; }, WT, sm);
+    launch_pair_kernel(t, k_pair_ww_tile<true>, k_pair_ww_tile_batch<true>,
+                       [&](const SysView& v) { return v.nw && eww(v) ? ww_tile_blocks(v) : 0; }, WT, sm);
+    launch_pair_kernel(t, k_pair_ww_tile<false>, k_pair_ww_tile_batch<false>,
+                       [&](const SysView& v) { return v.nw && !eww(v) ? ww_tile_blocks(v) : 0; }, WT, sm);
 }
 
 void launch_pairs_water(const Target& t, bool energy) {
@@ -848,16 +834,16 @@ void launch_pairs_water(const Target& t, bool energy) {
 void launch_pairs_ws(const Target& t, bool energy) {
     auto ws = [](const SysView& v) { return v.nw && v.na ? pair_blocks_ws(v) : 0; };
     const bool al = any_alch(t);
-    if (energy && al) t.launch(k_pair_ws<true, true>, k_pair_ws_batch<true, true>, ws, PT, 0);
-    else if (energy) t.launch(k_pair_ws<true, false>, k_pair_ws_batch<true, false>, ws, PT, 0);
-    else if (al) t.launch(k_pair_ws<false, true>, k_pair_ws_batch<false, true>, ws, PT, 0);
-    else t.launch(k_pair_ws<false, false>, k_pair_ws_batch<false, false>, ws, PT, 0);
+    if (energy && al) launch_pair_kernel(t, k_pair_ws<true, true>, k_pair_ws_batch<true, true>, ws, PT, 0);
+    else if (energy) launch_pair_kernel(t, k_pair_ws<true, false>, k_pair_ws_batch<true, false>, ws, PT, 0);
+    else if (al) launch_pair_kernel(t, k_pair_ws<false, true>, k_pair_ws_batch<false, true>, ws, PT, 0);
+    else launch_pair_kernel(t, k_pair_ws<false, false>, k_pair_ws_batch<false, false>, ws, PT, 0);
 }
 
 void launch_pair14(const Target& t, bool energy) {
     auto g = [](const SysView& v) { return v.n14 ? pair14_blocks(v) : 0; };
-    if (energy) t.launch(k_pair14<true>, k_pair14_batch<true>, g, 256, 0);
-    else t.launch(k_pair14<false>, k_pair14_batch<false>, g, 256, 0);
+    if (energy) launch_pair_kernel(t, k_pair14<true>, k_pair14_batch<true>, g, 256, 0);
+    else launch_pair_kernel(t, k_pair14<false>, k_pair14_batch<false>, g, 256, 0);
 }
 
 }  // namespace dyn

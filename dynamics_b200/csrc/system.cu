@@ -88,8 +88,7 @@ uint32_t ww_chunk_for(const SysView& v, const dyn_config_t* cfg, int ctas) {
     cudaDeviceGetAttribute(&smem_blk, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     size_t per_cta = smem_sm > 6144 * ctas ? (size_t)smem_sm / ctas - 6144 : 48 * 1024;
     per_cta = std::min<size_t>(per_cta, smem_blk > 0 ? (size_t)smem_blk : per_cta);
-    const uint32_t fit =
-        (uint32_t)((per_cta - 12 * sizeof(int)) / (4 * sizeof(float4) + 13 * sizeof(int))) / 32 * 32;
+    const uint32_t fit = (uint32_t)(per_cta / WW_CHUNK_BYTES) / 32 * 32;
     uint32_t chunk = std::max<uint32_t>(32u, std::min<uint32_t>(fit, (v.cap_union + 31) / 32 * 32));
     if (cfg->ww_union_chunk) chunk = std::max<uint32_t>(32u, std::min<uint32_t>(chunk, cfg->ww_union_chunk / 32 * 32));
     return chunk;
@@ -299,7 +298,6 @@ int check_scalars(dyn_sys_s* h) {
         return dyn::fail(DYN_ERR_UNSUPPORTED, "cluster list capacity exceeded (list length " +
                                                   std::to_string(h->h_sc->overflow) + ")");
     if (h->h_sc->nonfinite) return dyn::fail(DYN_ERR_NONFINITE, "non-finite coordinates or forces");
-    if (h->h_sc->timeout) return dyn::fail(DYN_ERR_TIMEOUT, "a bounded device wait gave up");
     return DYN_OK;
 }
 }  // namespace dyn
@@ -471,7 +469,8 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     v.total_mass = (double)v.nw * (double)OPC_MASS_MOL;
     for (uint32_t a = 0; a < v.na && d->atom_mass; ++a) v.total_mass += (double)d->atom_mass[a];
     // parameters
-    v.rc = rc; v.rc2 = rc * rc; v.ljc2 = ljc * ljc; v.alpha = cfg->ewald_alpha;
+    v.rc = rc; v.alpha = cfg->ewald_alpha;
+    v.pp.rc2 = rc * rc; v.pp.ljc2 = ljc * ljc; v.pp.alpha = cfg->ewald_alpha;
     v.buffer = cfg->list_buffer;
     v.r_ww = std::max(ljc, rc + 2.0f * OPC_SITE_REACH) + v.buffer;
     v.r_ws = std::max(ljc, rc + OPC_SITE_REACH) + v.buffer;
@@ -495,7 +494,7 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     // column grid: edge close to that of a cube holding one 32-water group
     const double vol = (double)ext[0] * ext[1] * ext[2];
     const double dens = (double)std::max<uint32_t>(1u, v.nw + v.na / 3) / vol;
-    const double edge = std::cbrt((double)GRPW / dens);
+        const double edge = std::cbrt((double)GRPW / dens);
     v.ncx = std::max(1u, (uint32_t)std::floor(ext[0] / edge));
     v.ncy = std::max(1u, (uint32_t)std::floor(ext[1] / edge));
     v.ncol = v.ncx * v.ncy;
@@ -553,13 +552,14 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
         // several chunks, so this is only the list-build capacity
         v.cap_union = std::min<uint32_t>((uint32_t)(2.8 * mink(ag) * dl) + 64, 65534u);
         v.cap_union = std::min<uint32_t>(v.cap_union, v.nw_cap);
-        // shared-memory chunk of the water-water kernel: three CTAs per SM
-        v.union_chunk = ww_chunk_for(v, cfg, 3);
-        v.cap_run = v.cap_union;  // a run per union water at worst
-        // fewer water groups than SMs: several CTAs share each group's entries
         int dev = 0, n_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+        // shared-memory chunk of the water-water kernel: sized for three CTAs
+        // per SM, or for two where all groups are resident then, as fewer
+        // unions are cut into chunks (256 groups: 39 us against 46)
+        v.union_chunk = ww_chunk_for(v, cfg, v.ngrp_cap <= 2u * (uint32_t)std::max(n_sm, 1) ? 2 : 3);
+        // fewer water groups than SMs: each is cut into several parts
         v.ww_split = v.ngrp_cap ? std::max<uint32_t>(1u, std::min<uint32_t>(8u, ((uint32_t)std::max(n_sm, 1) +
                                                                                v.ngrp_cap - 1) / v.ngrp_cap))
                                 : 1u;
@@ -594,8 +594,8 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
             const double r = std::sqrt(z), x = a * r;
             return (c * std::exp(-x * x) / r - std::erf(x) / z) / r;
         };
-        cheb_poly<NPOLY_G>(g, (double)v.rc * (double)v.rc, v.poly_g);
-        v.two_over_rc2 = (float)(2.0 / ((double)v.rc * (double)v.rc));
+        cheb_poly<NPOLY_G>(g, (double)v.rc * (double)v.rc, v.pp.poly_g);
+        v.pp.two_over_rc2 = (float)(2.0 / ((double)v.rc * (double)v.rc));
     }
     // mixed lists: every cluster while that stays small (sparse atoms such as
     // ions form clusters with wide bounding boxes), else the estimate
@@ -656,13 +656,12 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     TRY(dev_alloc(h, &v.gbb_c, v.ngrp_cap));
     TRY(dev_alloc(h, &v.gbb_h, v.ngrp_cap));
     TRY(dev_alloc(h, &v.tile_j, (size_t)v.ngrp_cap * v.cap_tile));
-    TRY(dev_alloc(h, &v.grp_nrun, v.ngrp_cap));
     TRY(dev_alloc(h, &v.grp_nloc, v.ngrp_cap));
-    TRY(dev_alloc(h, &v.grp_run, (size_t)v.ngrp_cap * v.cap_run));
     TRY(dev_alloc(h, &v.wnb_n, v.nw_cap));
     TRY(dev_alloc(h, &v.wnb, (size_t)v.nw_cap * v.cap_nb));
     TRY(dev_alloc(h, &v.winb_n, v.nw_cap));
     TRY(dev_alloc(h, &v.winb, (size_t)v.nw_cap * v.cap_nb));
+    TRY(dev_alloc(h, &v.winb_cut, (size_t)v.nw_cap * WW_SPLIT_MAX));
     TRY(dev_alloc(h, &v.wprune, v.nw_cap));
     TRY(dev_alloc(h, &v.grp_uslot, (size_t)v.ngrp_cap * v.cap_union));
     TRY(dev_alloc(h, &v.ws_n, v.nwclus_cap));
@@ -1455,11 +1454,6 @@ int evaluate_forces(dyn_sys_s* h) { return evaluate_forces_now(h); }
 
 namespace dyn {
 void energies_of(dyn_sys_s* h, dyn_energies_t* e) { fill_energies(h, e); }
-
-void set_ww_split(dyn_sys_s* h, uint32_t split) {
-    h->v.ww_split = std::max(1u, std::min(8u, split));
-    set_block_counts(h->v);
-}
 
 void set_batch_member(dyn_sys_s* h) {
     h->batch_member = true;
