@@ -152,9 +152,10 @@ struct SysView {
     uint32_t* wcol; uint32_t* acol;             // column of each water / atom
     // cluster bounding boxes (center xyz, half extent xyz)
     float4* wbb_c; float4* wbb_h; float4* abb_c; float4* abb_h;
-    // cluster lists (fixed capacity per i cluster): water cluster -> atom
-    // clusters, atom cluster -> atom clusters (cj >= ci) with masks; work
-    // items {i cluster, first entry} of ch_mix (1..32) list entries, in i order
+    // lists of the atom clusters (fixed capacity each): the waters within the
+    // list radius of any atom of the cluster (slots, ascending), and the atom
+    // clusters (cj >= ci) with masks; work items {cluster, first entry} of 32
+    // waters or ch_mix (1..32) clusters, in cluster order
     uint32_t cap_ws, cap_ss, ch_mix;
     uint32_t* ws_n; uint32_t* ws_j;
     uint32_t* ss_n; uint32_t* ss_j; unsigned long long* ss_mask;

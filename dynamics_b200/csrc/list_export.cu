@@ -2,8 +2,8 @@
 //
 // The pair kernels never see a flat pair list: water-water pairs come from
 // per-water lists of indices into a water group's union of j-waters,
-// water-atom and atom-atom pairs from cluster-pair lists (the latter with
-// 64-bit interaction masks).  This expands the lists exactly as the kernels
+// water-atom pairs from the atom clusters' lists of waters, atom-atom pairs
+// from cluster-pair lists with 64-bit interaction masks.  This expands the lists exactly as the kernels
 // walk them into pairs of original indices (water ids in the order the
 // system was created, atom indices), so that a test can check that every
 // pair inside the cutoff is covered (src/neighbors.rs:102-281 holds every
@@ -58,25 +58,22 @@ int ww_pairs(const SysView& v, const Scalars& sc, std::vector<uint32_t>& out) {
     return DYN_OK;
 }
 
-// water-atom: every (water, atom) of the water-cluster x atom-cluster pairs
+// water-atom: every atom of a cluster with every water of its list
 int ws_pairs(const SysView& v, const Scalars& sc, std::vector<uint32_t>& out) {
     std::vector<uint32_t> wid, sidx, n, j;
     TRY_D2H(wid, v.wid, v.nw_cap);
     TRY_D2H(sidx, v.sidx, v.na_cap);
-    TRY_D2H(n, v.ws_n, sc.n_wclus);
-    TRY_D2H(j, v.ws_j, (size_t)sc.n_wclus * v.cap_ws);
-    for (uint32_t ci = 0; ci < sc.n_wclus; ++ci)
+    TRY_D2H(n, v.ws_n, sc.n_aclus);
+    TRY_D2H(j, v.ws_j, (size_t)sc.n_aclus * v.cap_ws);
+    for (uint32_t ci = 0; ci < sc.n_aclus; ++ci)
         for (uint32_t k = 0; k < n[ci]; ++k) {
-            const uint32_t cj = j[(size_t)ci * v.cap_ws + k];
-            for (uint32_t ii = 0; ii < WCL; ++ii) {
-                const uint32_t w = wid[ci * WCL + ii];
-                if (w == INVALID_ID) continue;
-                for (uint32_t jj = 0; jj < ACL; ++jj) {
-                    const uint32_t a = sidx[(size_t)cj * ACL + jj];
-                    if (a == INVALID_ID) continue;
-                    out.push_back(w);
-                    out.push_back(a);
-                }
+            const uint32_t w = wid[j[(size_t)ci * v.cap_ws + k]];
+            if (w == INVALID_ID) continue;
+            for (uint32_t jj = 0; jj < ACL; ++jj) {
+                const uint32_t a = sidx[(size_t)ci * ACL + jj];
+                if (a == INVALID_ID) continue;
+                out.push_back(w);
+                out.push_back(a);
             }
         }
     return DYN_OK;

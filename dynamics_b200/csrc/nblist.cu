@@ -413,10 +413,9 @@ __device__ __forceinline__ void clear_excluded(const SysView& v, uint32_t ci, ui
     }
 }
 
-// One warp per i-cluster.  MODE 1: water i-clusters against atom
-// j-clusters; MODE 3: atom i-clusters against atom j-clusters with cj >= ci
-// (each cluster pair once), with the interaction mask of the cluster pair
-// (jj > ii on the diagonal, exclusions and pairs of two static atoms
+// Atom-atom cluster pairs: one warp per i-cluster, against the clusters with
+// cj >= ci (each cluster pair once), with the interaction mask of the cluster
+// pair (jj > ii on the diagonal, exclusions and pairs of two static atoms
 // removed).  LU blocks of 32 candidates are tested per turn, so that their
 // boxes' loads are in flight together.  A lane makes its hit's mask as the
 // product of the two clusters' valid-atom bits (one byte per i-atom); the
@@ -424,26 +423,19 @@ __device__ __forceinline__ void clear_excluded(const SysView& v, uint32_t ci, ui
 // the 64 pairs of every hit were decided by binary searches in the exclusion
 // lists.
 constexpr int LU = 4;
-DYN_KERNEL_T((int MODE), (MODE), , k_list, (, bool force), (, force)) {
+DYN_KERNEL(, k_list_ss, (, bool force), (, force)) {
     if (!rebuild_on(v, force)) return;
     const BoxDev b = *v.box;
     const int lane = threadIdx.x & 31;
     const uint32_t ci = (bk.idx * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t ni = MODE == 1 ? v.sc->n_wclus : v.sc->n_aclus;
-    const uint32_t nj = v.sc->n_aclus;
-    if (ci >= ni) return;
-    const float4* bcj = v.abb_c;
-    const float4* bhj = v.abb_h;
-    const float r = MODE == 3 ? v.r_ss : v.r_ws;
-    const float r2 = r * r;
-    const uint32_t cap = MODE == 1 ? v.cap_ws : v.cap_ss;
-    uint32_t* out = MODE == 1 ? v.ws_j : v.ss_j;
-    uint32_t* outn = MODE == 1 ? v.ws_n : v.ss_n;
-    const float4 c0 = MODE == 1 ? v.wbb_c[ci] : v.abb_c[ci];
-    const float4 h0 = MODE == 1 ? v.wbb_h[ci] : v.abb_h[ci];
+    const uint32_t nc = v.sc->n_aclus;
+    if (ci >= nc) return;
+    const float r2 = v.r_ss * v.r_ss;
+    const uint32_t cap = v.cap_ss;
+    const float4 c0 = v.abb_c[ci], h0 = v.abb_h[ci];
     // a byte per i-atom: 1 where the slot holds an atom, and where that atom is static
     unsigned long long vi = 0ull, si = 0ull;
-    if (MODE == 3) {
+    {
         const uint32_t a = lane < ACL ? v.sidx[ci * ACL + lane] : INVALID_ID;
         const bool st = a != INVALID_ID && v.astatic && v.astatic[a];
         const uint32_t mv = __ballot_sync(0xffffffffu, a != INVALID_ID), ms = __ballot_sync(0xffffffffu, st);
@@ -454,12 +446,12 @@ DYN_KERNEL_T((int MODE), (MODE), , k_list, (, bool force), (, force)) {
         }
     }
     uint32_t cnt = 0;
-    for (uint32_t jb = MODE == 3 ? (ci & ~31u) : 0u; jb < nj; jb += 32 * LU) {
+    for (uint32_t jb = ci & ~31u; jb < nc; jb += 32 * LU) {
         bool hit[LU];
 #pragma unroll
         for (int u = 0; u < LU; ++u) {
             const uint32_t cj = jb + 32 * u + lane;
-            hit[u] = cj < nj && (MODE != 3 || cj >= ci) && bb_dist2(c0, h0, bcj[cj], bhj[cj], b) < r2;
+            hit[u] = cj < nc && cj >= ci && bb_dist2(c0, h0, v.abb_c[cj], v.abb_h[cj], b) < r2;
         }
 #pragma unroll
         for (int u = 0; u < LU; ++u) {
@@ -468,58 +460,152 @@ DYN_KERNEL_T((int MODE), (MODE), , k_list, (, bool force), (, force)) {
             const uint32_t k = cnt + __popc(m & ((1u << lane) - 1u));
             cnt += __popc(m);
             if (!hit[u] || k >= cap) continue;
-            out[(size_t)ci * cap + k] = cj;
-            if (MODE == 3) {
-                const uint4* sj = reinterpret_cast<const uint4*>(v.sidx + (size_t)cj * ACL);
-                const uint4 s0 = sj[0], s1 = sj[1];
-                const uint32_t aj[ACL] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-                uint32_t vj = 0;
+            v.ss_j[(size_t)ci * cap + k] = cj;
+            const uint4* sj = reinterpret_cast<const uint4*>(v.sidx + (size_t)cj * ACL);
+            const uint4 s0 = sj[0], s1 = sj[1];
+            const uint32_t aj[ACL] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+            uint32_t vj = 0;
 #pragma unroll
-                for (int jj = 0; jj < ACL; ++jj) vj |= aj[jj] != INVALID_ID ? 1u << jj : 0u;
-                unsigned long long mk = vi * vj;  // byte ii: the j-atoms, where i-atom ii exists
-                if (si) {
-                    uint32_t sj8 = 0;
+            for (int jj = 0; jj < ACL; ++jj) vj |= aj[jj] != INVALID_ID ? 1u << jj : 0u;
+            unsigned long long mk = vi * vj;  // byte ii: the j-atoms, where i-atom ii exists
+            if (si) {
+                uint32_t sj8 = 0;
 #pragma unroll
-                    for (int jj = 0; jj < ACL; ++jj)
-                        if (aj[jj] != INVALID_ID && v.astatic[aj[jj]]) sj8 |= 1u << jj;
-                    mk &= ~(si * sj8);
-                }
-                if (cj == ci) mk &= 0x0080C0E0F0F8FCFEull;  // byte ii: the bits jj > ii
-                v.ss_mask[(size_t)ci * cap + k] = mk;
+                for (int jj = 0; jj < ACL; ++jj)
+                    if (aj[jj] != INVALID_ID && v.astatic[aj[jj]]) sj8 |= 1u << jj;
+                mk &= ~(si * sj8);
             }
+            if (cj == ci) mk &= 0x0080C0E0F0F8FCFEull;  // byte ii: the bits jj > ii
+            v.ss_mask[(size_t)ci * cap + k] = mk;
         }
     }
     const uint32_t n = min(cnt, cap);
-    if (MODE == 3 && v.ex_off) {
+    if (v.ex_off) {
         __syncwarp();  // the list and the masks are written
         clear_excluded(v, ci, n, lane);
     }
     if (lane == 0) {
-        outn[ci] = n;
+        v.ss_n[ci] = n;
         if (cnt > cap) atomicMax(&v.sc->overflow, cnt);
         atomicAdd(&v.sc->list_pairs, (unsigned long long)n);
     }
 }
 
-// Work items of the atom pair kernels: for every i-cluster (in order) one
-// item per ch_mix entries of its list, {cluster, first entry}.  Block 0 the
-// water-atom items, block 1 the atom-atom ones; an exclusive scan of the
-// per-cluster item counts, tile by tile.
+// The waters of every atom cluster: those whose O lies within the list radius
+// of any of the cluster's atoms, ascending by slot; a CTA per cluster.  Of
+// every WLC water clusters, those whose box meets the atom cluster's (four
+// boxes in flight per thread) are tested water by water, two waters per
+// thread.  Bound by latency; 750 clusters against 3,000 water clusters:
+// 32 us (53 with one box and one water per thread and turn).
+constexpr int WLT = 256, WLU = 4, WLW = 2;
+constexpr int WLC = WLT * WLU;
+DYN_KERNEL(__launch_bounds__(WLT), k_list_ws, (, bool force), (, force)) {
+    if (!rebuild_on(v, force)) return;
+    const BoxDev b = *v.box;
+    const float r2 = v.r_ws * v.r_ws;
+    const int tid = threadIdx.x, lane = tid & 31, wid_ = tid >> 5;
+    constexpr int NWP = WLT / 32;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t nwc = v.sc->n_wclus, nac = v.sc->n_aclus;
+    __shared__ float4 ap[ACL];
+    __shared__ uint32_t cl[WLC];       // water clusters met by the box
+    __shared__ uint32_t wt[WLU][NWP];
+    // where this warp's hits of pass u start after base; base moves past all
+    auto place = [&](uint32_t& base, int u) {
+        uint32_t at = base;
+#pragma unroll
+        for (int w = 0; w < NWP; ++w) {
+            if (w < wid_) at += wt[u][w];
+            base += wt[u][w];
+        }
+        return at;
+    };
+    for (uint32_t ci = bk.idx; ci < nac; ci += bk.cnt) {
+        if (tid < ACL) {
+            const float4 p = v.spos[ci * ACL + tid];
+            ap[tid] = make_float4(p.x, p.y, p.z, v.sidx[ci * ACL + tid] != INVALID_ID ? 1.f : 0.f);
+        }
+        const float4 c0 = v.abb_c[ci], h0 = v.abb_h[ci];
+        uint32_t* out = v.ws_j + (size_t)ci * v.cap_ws;
+        uint32_t cnt = 0;
+        for (uint32_t jb = 0; jb < nwc; jb += WLC) {
+            uint32_t m[WLU];
+#pragma unroll
+            for (int u = 0; u < WLU; ++u) {
+                const uint32_t cj = jb + u * WLT + tid;
+                m[u] = __ballot_sync(0xffffffffu, cj < nwc && bb_dist2(c0, h0, v.wbb_c[cj], v.wbb_h[cj], b) < r2);
+                if (lane == 0) wt[u][wid_] = __popc(m[u]);
+            }
+            __syncthreads();
+            uint32_t nc = 0;
+#pragma unroll
+            for (int u = 0; u < WLU; ++u) {
+                const uint32_t at = place(nc, u);
+                if ((m[u] >> lane) & 1u) cl[at + __popc(m[u] & lt)] = jb + u * WLT + tid;
+            }
+            __syncthreads();
+            for (uint32_t k0 = 0; k0 < nc * WCL; k0 += WLT * WLW) {
+                uint32_t slot[WLW], mn[WLW];
+                bool near[WLW];
+#pragma unroll
+                for (int u = 0; u < WLW; ++u) {
+                    const uint32_t k = k0 + u * WLT + tid;
+                    const bool in = k < nc * WCL;
+                    slot[u] = in ? cl[k / WCL] * WCL + (k % WCL) : 0u;
+                    near[u] = in && v.wid[slot[u]] != INVALID_ID;
+                }
+#pragma unroll
+                for (int u = 0; u < WLW; ++u) {
+                    const float3 o = xyz(v.wpos[4 * slot[u]]);
+                    bool any = false;
+#pragma unroll
+                    for (int i = 0; i < ACL; ++i) {
+                        const float4 q = ap[i];
+                        const float3 d = min_image_fast(o - xyz(q), b);
+                        any = any || (q.w != 0.f && dot3(d, d) < r2);
+                    }
+                    near[u] = near[u] && any;
+                    mn[u] = __ballot_sync(0xffffffffu, near[u]);
+                    if (lane == 0) wt[u][wid_] = __popc(mn[u]);
+                }
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < WLW; ++u) {
+                    const uint32_t pos = place(cnt, u) + __popc(mn[u] & lt);
+                    if (near[u] && pos < v.cap_ws) out[pos] = slot[u];
+                }
+                __syncthreads();  // the counts are refilled
+            }
+        }
+        if (tid == 0) {
+            v.ws_n[ci] = min(cnt, v.cap_ws);
+            if (cnt > v.cap_ws) atomicMax(&v.sc->overflow, cnt);
+            atomicAdd(&v.sc->list_pairs, (unsigned long long)min(cnt, v.cap_ws));
+        }
+        __syncthreads();  // the atoms are refilled
+    }
+}
+
+// Work items of the atom pair kernels: for every atom cluster (in order) one
+// item per 32 waters or ch_mix clusters of its list, {cluster, first
+// entry}.  Block 0 the water-atom items, block 1 the atom-atom ones; an
+// exclusive scan of the per-cluster item counts, tile by tile.
 constexpr int IT_T = 1024;
 DYN_KERNEL(__launch_bounds__(IT_T), k_items, (, bool force), (, force)) {
     if (!rebuild_on(v, force)) return;
     const bool ws = bk.idx == 0;
     if (ws && !v.nw) return;
-    const uint32_t ni = ws ? v.sc->n_wclus : v.sc->n_aclus;
+    const uint32_t ni = v.sc->n_aclus;
     const uint32_t* cnt = ws ? v.ws_n : v.ss_n;
     uint2* items = ws ? v.ws_item : v.ss_item;
     const uint32_t icap = ws ? v.ws_item_cap : v.ss_item_cap;
+    const uint32_t per = ws ? 32u : v.ch_mix;
     __shared__ uint32_t wsum[IT_T / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     uint32_t base = 0;
     for (uint32_t c0 = 0; c0 < ni; c0 += IT_T) {
         const uint32_t c = c0 + threadIdx.x;
-        const uint32_t k = c < ni ? (cnt[c] + v.ch_mix - 1) / v.ch_mix : 0u;
+        const uint32_t k = c < ni ? (cnt[c] + per - 1) / per : 0u;
         uint32_t x = k;  // inclusive scan inside the warp
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -540,7 +626,7 @@ DYN_KERNEL(__launch_bounds__(IT_T), k_items, (, bool force), (, force)) {
         __syncthreads();
         const uint32_t off = base + (w ? wsum[w - 1] : 0u) + x - k;
         for (uint32_t t = 0; t < k; ++t)
-            if (off + t < icap) items[off + t] = make_uint2(c, t * v.ch_mix);
+            if (off + t < icap) items[off + t] = make_uint2(c, t * per);
         base += wsum[IT_T / 32 - 1];
         __syncthreads();
     }
@@ -878,10 +964,10 @@ void launch_rebuild(const Target& t, bool force) {
     const int LT = 128;  // 4 warps per block, one i-cluster per warp
     t.launch(k_group_union, k_group_union_batch,
              [](const SysView& v) { return v.nw ? (int)std::min<uint32_t>(v.ngrp_cap, 148 * 8) : 0; }, UT, 0, force);
-    t.launch(k_list<1>, k_list_batch<1>,
-             [](const SysView& v) { return v.nw && v.na ? nblocks((uint64_t)v.nwclus_cap * 32, 128, 1 << 30) : 0; },
-             LT, 0, force);
-    t.launch(k_list<3>, k_list_batch<3>,
+    t.launch(k_list_ws, k_list_ws_batch,
+             [](const SysView& v) { return v.nw && v.na ? (int)std::min<uint32_t>(v.naclus_cap, 148 * 8) : 0; }, WLT, 0,
+             force);
+    t.launch(k_list_ss, k_list_ss_batch,
              [](const SysView& v) { return v.na ? nblocks((uint64_t)v.naclus_cap * 32, 128, 1 << 30) : 0; }, LT, 0,
              force);
     t.launch(k_items, k_items_batch, [](const SysView& v) { return v.na ? 2 : 0; }, IT_T, 0, force);

@@ -7,21 +7,19 @@
 // between charged sites, 1-2/1-3 exclusions, no intra-water pairs; 1-4 pairs
 // are excluded here and evaluated (scaled) by k_pair14.
 //
-// Work decomposition.  Water-water: one CTA per
-// 32-water i-group, j sites staged in shared memory, the group's molecule
-// lists dealt out over the threads (k_pair_ww_tile).  Atom-water and atom-atom
-// (half lists: every pair once): one warp per work item (an 8-body
-// i-cluster and up to ch_mix entries of its list); lane = (ii, jq) with
-// ii = lane & 7 and jq = lane >> 3 evaluates i-body ii against j-atoms jq and
-// jq + 4 of every j-cluster in the item.  Water pairs are
-// handled as molecule pairs: one min-image shift from the O-O vector serves
-// all site pairs, valid because the cutoff plus twice the O-H reach is below
-// half the box.  i-forces stay in registers over the whole list, are reduced
-// over the lanes sharing an i-body with shuffles and written once as int64
-// fixed point; the water-water kernel stores (first writer), the others add,
-// and j-side forces go out as integer atomics after a reduce-scatter over
-// the lanes of a j-body.  Integer sums do not depend on order, so the
-// result is deterministic.
+// Work decomposition.  Water-water: one CTA per 32-water i-group (or part of
+// one), j sites staged in shared memory, the group's molecule lists dealt out
+// over the threads (k_pair_ww_tile).  Water-atom: one warp per atom cluster
+// and batch of the waters listed for it, a lane per water (k_pair_ws).
+// Atom-atom: one warp per work item (an 8-atom i-cluster and up to ch_mix
+// entries of its list); lane = (ii, jq) with ii = lane & 7 and jq = lane >> 3
+// evaluates i-atom ii against j-atoms jq and jq + 4 of every j-cluster in the
+// item (k_pair_ss).  All lists hold every pair once.  A water is moved as a
+// whole: one min-image shift from its O serves all its sites, valid because
+// the cutoff plus twice the O-H reach is below half the box.  Forces are
+// summed in float32 registers as far as a thread's work goes and added to the
+// int64 fixed-point accumulators with reductions; integer sums do not depend
+// on order, so the result is deterministic.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -493,131 +491,104 @@ __device__ __forceinline__ JAtoms load_jatoms(const SysView& v, uint32_t cj, int
 }
 
 // ---------------------------------------------------------------------------
-// water(i) - atom(j), each pair once.  One warp per work item (a water
-// i-cluster and ch_mix entries of its atom-cluster list); the list entries
-// are read once per item (one per lane) and the next entry's j-atoms are
-// loaded while the current one is evaluated.  The water forces stay in
-// registers over the item; the j-atom forces (the opposite of the pair
-// forces) are reduce-scattered over the 8 water lanes of a j-group and added
-// with integer atomics (24 per entry).
+// water - atom, each pair once.  One warp per work item: an atom cluster (up
+// to 8 atoms) and 32 of the waters listed within the list radius of any of its
+// atoms.  A lane takes one water and evaluates it against the cluster's atoms
+// in turn (their data is the same for all lanes: one broadcast load each), so
+// that the lanes' work is the listed waters and not the pairs of two bounding
+// boxes.  The water's forces stay in registers over the atoms and are added
+// once (12 int64 reductions); each lane keeps its share of the atoms' forces
+// in shared memory (24 sums per lane, no conflicts), added up over the lanes
+// in a fixed order at the end, one lane per component.  An atom beyond the
+// cutoff plus the O-H reach of all 32 waters is skipped by a vote.
+//
+// Bound by issue (the energies take about as much as the forces, on every
+// step by default) at 16 warps per SM.  24,000 waters and 5,000 atoms: 40 us
+// and 18 M warp instructions, against 74 us and 40 M for pairs of an 8-water
+// and an 8-atom cluster (few of whose 64 pairs are in range: the water
+// clusters are 2.7 A thin in a column 10.8 A wide); 8,000 waters and 640 atoms
+// 28 -> 16 us, 2,900 and 510 21 -> 15.  Two or four batches of 32 waters per
+// item 43 and 45 us; 5 and 6 CTAs per SM 46 and 43.
 // ---------------------------------------------------------------------------
 DYN_KERNEL_T((bool ENERGY, bool ALCH), (ENERGY, ALCH), __launch_bounds__(PT, 4), k_pair_ws, (, const PairParams P), (, P)) {
-    const int lane = threadIdx.x & 31;
-    const int ii = lane & 7, jq = lane >> 3;
+    __shared__ float fa[PT / 32][3 * ACL][32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const uint32_t nwarps = (bk.cnt * blockDim.x) >> 5;
     const uint32_t nit = v.sc->n_ws_items;
-    const uint32_t first_single = v.sc->a_sparse_base / ACL;  // first single-atom cluster
     const BoxDev b = *v.box;
     const float ljc2 = P.ljc2;
-    double el = 0.0, ec = 0.0, ew = 0.0, dh = 0.0;
+    double el = 0.0, ec = 0.0, dh = 0.0;
+    Acc3 a{0.0, 0.0, 0.f, 0.0};
     for (uint32_t it = ((bk.idx * blockDim.x + threadIdx.x) >> 5); it < nit; it += nwarps) {
         const uint2 item = v.ws_item[it];
         const uint32_t ci = item.x, k0 = item.y;
-        const uint32_t n = min(v.ws_n[ci], k0 + v.ch_mix) - k0;
-        const uint32_t si = ci * WCL + ii;
-        const bool vi = v.wid[si] != INVALID_ID;
-        const float3 iO = xyz(v.wpos[4 * si + 0]), iH0 = xyz(v.wpos[4 * si + 1]);
-        const float3 iH1 = xyz(v.wpos[4 * si + 2]), iM = xyz(v.wpos[4 * si + 3]);
-        float3 fO = f3(0, 0, 0), fH0 = fO, fH1 = fO, fM = fO;
-        Acc3 a{0.0, 0.0, 0.f, 0.0};
-        const uint32_t my_j = (uint32_t)lane < n ? v.ws_j[(size_t)ci * v.cap_ws + k0 + lane] : 0u;
-        // Single-atom clusters (ions) come last in every list.  Four of them
-        // are taken per iteration, one per lane group jq (its atom in the
-        // h = 0 slot), instead of one cluster with seven empty slots.
-        auto load_at = [&](uint32_t k) -> JAtoms {
-            const uint32_t c0 = __shfl_sync(0xffffffffu, my_j, k);
-            const uint32_t kk = k + (uint32_t)jq;
-            const uint32_t cq = __shfl_sync(0xffffffffu, my_j, kk < n ? kk : k);
-            if (c0 < first_single) return load_jatoms(v, c0, jq);
-            const uint32_t sq = cq * ACL;
-            return JAtoms{v.spos[sq], make_float4(0.f, 0.f, 0.f, 0.f), v.slj[sq], make_float2(0.f, 0.f),
-                          kk < n ? v.sidx[sq] : INVALID_ID, INVALID_ID};
-        };
-        auto advance = [&](uint32_t k) -> uint32_t {
-            return __shfl_sync(0xffffffffu, my_j, k) < first_single ? 1u : 4u;
-        };
-        JAtoms nx = load_at(0);
-        for (uint32_t k = 0; k < n;) {
-            const JAtoms cur = nx;
-            k += advance(k);
-            if (k < n) nx = load_at(k);
-            // the cluster boxes met within r_ws; skip the half (atoms 0-3 or
-            // 4-7) of the entry where no lane's water O lies within cutoff +
-            // O-H reach of an atom
-            bool near0, near1;
-            {
-                const float r2 = v.r_ws_skip2;
-                bool n0 = false, n1 = false;
-                if (vi && cur.a0 != INVALID_ID) {
-                    const float3 d = min_image_fast(iO - xyz(cur.p0), b);
-                    n0 = dot3(d, d) < r2;
-                }
-                if (vi && cur.a1 != INVALID_ID) {
-                    const float3 d = min_image_fast(iO - xyz(cur.p1), b);
-                    n1 = dot3(d, d) < r2;
-                }
-                near0 = __any_sync(0xffffffffu, n0);
-                near1 = __any_sync(0xffffffffu, n1);
-                if (!near0 && !near1) continue;
-            }
-            float jf[8];
+        const bool vi = k0 + lane < v.ws_n[ci];
+        const uint32_t s = v.ws_j[(size_t)ci * v.cap_ws + k0 + (vi ? lane : 0)];
+        const uint32_t ai = lane < ACL ? v.sidx[ci * ACL + lane] : INVALID_ID;
+        const uint32_t am = __ballot_sync(0xffffffffu, ai != INVALID_ID);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float4 pj = h ? cur.p1 : cur.p0;
-                const float2 lj_j = h ? cur.l1 : cur.l0;
-                const uint32_t aj = h ? cur.a1 : cur.a0;
-                float3 fo = f3(0, 0, 0), f0 = fo, f1 = fo, fm = fo;
-                if ((h ? near1 : near0) && vi && aj != INVALID_ID) {
-                    const float3 jp = xyz(pj);
-                    // the atom moved by the shift once, then zero shift
-                    const float3 js = jp - shift_of(iO - jp, b), z0 = f3(0.f, 0.f, 0.f);
-                    const float sg = 0.5f * (OPC_O_SIGMA + lj_j.x);
-                    const float ep = sqrtf(OPC_O_EPS * lj_j.y);
-                    const double qe = (double)pj.w;
-                    if (ALCH && aj >= v.alch_lo && aj < v.alch_hi) {
-                        // a water and an atom of the alchemical molecule
-                        lj_soft<ENERGY>(iO, js, z0, sg, ep, ljc2, v.alch_ll, v.alch_dll, fo, a, dh);
-                        Acc3 t{0.0, 0.0, 0.f, 0.0};
-                        coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f0, t);
-                        coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f1, t);
-                        coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, P, fm, t);
-                        const float cs = v.alch_cs;
-                        f0 = f0 * cs; f1 = f1 * cs; fm = fm * cs;
-                        a.w = fmaf(cs, t.w, a.w);
-                        if (ENERGY) { a.e_c += (double)cs * t.e_c; dh += (double)v.alch_dcs * t.e_c; }
-                    } else {
-                        lj<ENERGY>(iO, js, z0, sg * sg, ep, ljc2, 1.0f, fo, a);
-                        coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f0, a);
-                        coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f1, a);
-                        coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, P, fm, a);
-                    }
-                }
-                fO = fO + fo; fH0 = fH0 + f0; fH1 = fH1 + f1; fM = fM + fm;
-                const float3 t = (fo + f0) + (f1 + fm);
-                jf[3 * h + 0] = -t.x; jf[3 * h + 1] = -t.y; jf[3 * h + 2] = -t.z;
+        for (int k = 0; k < 3 * ACL; ++k) fa[wp][k][lane] = 0.f;
+        const float3 iO = xyz(v.wpos[4 * s + 0]), iH0 = xyz(v.wpos[4 * s + 1]);
+        const float3 iH1 = xyz(v.wpos[4 * s + 2]), iM = xyz(v.wpos[4 * s + 3]);
+        float3 fO = f3(0, 0, 0), fH0 = fO, fH1 = fO, fM = fO;
+        for (uint32_t mm = am; mm; mm &= mm - 1u) {
+            const int k = __ffs(mm) - 1;
+            const float4 pj = v.spos[ci * ACL + k];
+            const float2 lj_j = v.slj[ci * ACL + k];
+            // the atom moved to the image nearest the water's O once
+            const float3 jp = xyz(pj), z0 = f3(0.f, 0.f, 0.f);
+            const float3 js = f3(fmaf(nearest_int(iO.x - jp.x, b.inv_ext[0]), b.ext[0], jp.x),
+                                 fmaf(nearest_int(iO.y - jp.y, b.inv_ext[1]), b.ext[1], jp.y),
+                                 fmaf(nearest_int(iO.z - jp.z, b.inv_ext[2]), b.ext[2], jp.z));
+            const float3 dO = iO - js;
+            if (!__any_sync(0xffffffffu, vi && dot3(dO, dO) < v.r_ws_skip2)) continue;
+            if (!vi) continue;
+            float3 fo = z0, f0 = z0, f1 = z0, fm = z0;
+            const float sg = 0.5f * (OPC_O_SIGMA + lj_j.x);
+            const float ep = sqrtf(OPC_O_EPS * lj_j.y);
+            const double qe = (double)pj.w;
+            const uint32_t aj = ALCH ? v.sidx[ci * ACL + k] : 0u;
+            if (ALCH && aj >= v.alch_lo && aj < v.alch_hi) {
+                // a water and an atom of the alchemical molecule
+                lj_soft<ENERGY>(iO, js, z0, sg, ep, ljc2, v.alch_ll, v.alch_dll, fo, a, dh);
+                Acc3 t{0.0, 0.0, 0.f, 0.0};
+                coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f0, t);
+                coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f1, t);
+                coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, P, fm, t);
+                const float cs = v.alch_cs;
+                f0 = f0 * cs; f1 = f1 * cs; fm = fm * cs;
+                a.w = fmaf(cs, t.w, a.w);
+                if (ENERGY) { a.e_c += (double)cs * t.e_c; dh += (double)v.alch_dcs * t.e_c; }
+            } else {
+                lj<ENERGY>(iO, js, z0, sg * sg, ep, ljc2, 1.0f, fo, a);
+                coul<ENERGY>(iH0, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f0, a);
+                coul<ENERGY>(iH1, js, z0, OPC_Q_H * pj.w, (double)OPC_Q_H * qe, P, f1, a);
+                coul<ENERGY>(iM, js, z0, OPC_Q_EP * pj.w, (double)OPC_Q_EP * qe, P, fm, a);
             }
-            jf[6] = 0.f; jf[7] = 0.f;
             a.flush_w();
-            // lane ii < 6 now holds component ii % 3 of the group's j-atom a0 (ii < 3) or a1
-            reduce_scatter8(jf, ii);
-            if (ii < 6) {
-                const uint32_t aj = ii < 3 ? cur.a0 : cur.a1;
-                if (aj != INVALID_ID) add_fix(v.aforce + 3 * (size_t)aj + ii % 3, jf[0]);
-            }
+            fO = fO + fo; fH0 = fH0 + f0; fH1 = fH1 + f1; fM = fM + fm;
+            const float3 t = (fo + f0) + (f1 + fm);
+            fa[wp][3 * k + 0][lane] -= t.x;
+            fa[wp][3 * k + 1][lane] -= t.y;
+            fa[wp][3 * k + 2][lane] -= t.z;
         }
-        fO = f3(red4(fO.x), red4(fO.y), red4(fO.z));
-        fH0 = f3(red4(fH0.x), red4(fH0.y), red4(fH0.z));
-        fH1 = f3(red4(fH1.x), red4(fH1.y), red4(fH1.z));
-        fM = f3(red4(fM.x), red4(fM.y), red4(fM.z));
-        if (jq == 0 && vi) {
-            long long* p = v.wforce + (size_t)si * 12;
+        if (vi) {
+            long long* p = v.wforce + (size_t)s * 12;
             add_fix3(p + 0, fO); add_fix3(p + 3, fH0); add_fix3(p + 6, fH1); add_fix3(p + 9, fM);
         }
-        if (ENERGY) { el += a.e_lj; ec += a.e_c; }
-        a.flush_w();
-        ew += a.wd;
+        __syncwarp();
+        // lane 3 k + c adds up component c of atom k (rotated: no bank conflicts)
+        const uint32_t at = __shfl_sync(0xffffffffu, ai, lane / 3);
+        if (lane < 3 * ACL && at != INVALID_ID) {
+            float f = 0.f;
+#pragma unroll 8
+            for (int j = 0; j < 32; ++j) f += fa[wp][lane][(lane + j) & 31];
+            add_fix(v.aforce + 3 * (size_t)at + lane % 3, f);
+        }
+        __syncwarp();
     }
-    write_partials_warp<ENERGY>(v, bk, REG_WS, el, ec, ew, dh);
+    if (ENERGY) { el = a.e_lj; ec = a.e_c; }
+    write_partials_warp<ENERGY>(v, bk, REG_WS, el, ec, a.wd, dh);
 }
 
 // ---------------------------------------------------------------------------

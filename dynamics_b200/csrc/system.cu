@@ -520,7 +520,7 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     }
     v.na_cap = round8(v.na - v.n_sparse + 8) + ACL * v.n_sparse;
     v.naclus_cap = v.na_cap / ACL;
-    v.max_blocks = 148 * 16;
+        v.max_blocks = 148 * 16;
 
     // list capacities from the cluster density, generous margin
     auto est = [&](double r, double cl_vol, uint32_t ncl) -> uint32_t {
@@ -603,10 +603,14 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
         if ((uint64_t)n_i * n_j <= (1ull << 24)) return std::max(1u, n_j);
         return est(r, vol_cl, n_j);
     };
-    v.cap_ws = (v.nw && v.na) ? cap_mixed(v.r_ws, acl_vol, v.nwclus_cap, v.naclus_cap) : 1;
+    // waters of an atom cluster: at worst 8 atoms far apart, each with the
+    // waters of its own sphere (half again as dense as the box or the liquid)
+    v.cap_ws = (v.nw && v.na)
+                   ? (uint32_t)std::min<double>(v.nw_cap, 8.0 * 1.5 * 4.0 / 3.0 * M_PI * std::pow((double)v.r_ws, 3) * dl + 64)
+                   : 1;
     v.cap_ss = v.na ? cap_mixed(v.r_ss, acl_vol, v.naclus_cap, v.naclus_cap) : 1;
-    v.ch_mix = cfg->pair_item_entries ? std::min(32u, cfg->pair_item_entries) : 8u;
-    v.ws_item_cap = v.nwclus_cap * ((v.cap_ws + v.ch_mix - 1) / v.ch_mix);
+    v.ch_mix = cfg->pair_item_entries ? std::min(32u, cfg->pair_item_entries) : 4u;
+    v.ws_item_cap = v.naclus_cap * ((v.cap_ws + 31u) / 32u);
     v.ss_item_cap = v.naclus_cap * ((v.cap_ss + v.ch_mix - 1) / v.ch_mix);
 
     // ---- allocations ----
@@ -664,8 +668,8 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     TRY(dev_alloc(h, &v.winb_cut, (size_t)v.nw_cap * WW_SPLIT_MAX));
     TRY(dev_alloc(h, &v.wprune, v.nw_cap));
     TRY(dev_alloc(h, &v.grp_uslot, (size_t)v.ngrp_cap * v.cap_union));
-    TRY(dev_alloc(h, &v.ws_n, v.nwclus_cap));
-    TRY(dev_alloc(h, &v.ws_j, (size_t)v.nwclus_cap * v.cap_ws));
+    TRY(dev_alloc(h, &v.ws_n, v.naclus_cap));
+    TRY(dev_alloc(h, &v.ws_j, (size_t)v.naclus_cap * v.cap_ws));
     TRY(dev_alloc(h, &v.ws_item, std::max(1u, v.ws_item_cap)));
     TRY(dev_alloc(h, &v.ss_item, std::max(1u, v.ss_item_cap)));
     TRY(dev_alloc(h, &v.ss_n, v.naclus_cap));

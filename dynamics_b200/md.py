@@ -110,8 +110,8 @@ class MdConfig:
     # charged sites per SPME grid brick before the overflow path; 0 =
     # automatic (results do not depend on it)
     spme_brick_cap: int = 0
-    # list entries per work item of the water-atom and atom-atom pair
-    # kernels (1..32); 0 = 8 (tuning knob only)
+    # list entries per work item of the atom-atom pair kernel (1..32);
+    # 0 = automatic (tuning knob only)
     pair_item_entries: int = 0
     # CTAs sharing one water group's list entries (1..8); 0 = automatic
     # (tuning knob only)

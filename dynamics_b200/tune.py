@@ -10,11 +10,10 @@ measurement, per size class of system, and cached:
   (shorter lists against more prunes);
 * ``ww_union_chunk``: the water-water kernel's shared-memory chunk (waters
   staged at a time; three CTAs per SM at the largest);
-* ``pair_item_entries``: list entries per work item of the water-atom and
-  atom-atom pair kernels (more items balance better, fewer amortise the
-  per-item loads);
-* ``ww_split``: CTAs sharing one water group's list entries (more CTAs
-  shorten the last wave, each stages the group's union again);
+* ``pair_item_entries``: list entries per work item of the atom-atom pair
+  kernel (more items balance better, fewer amortise the per-item loads);
+* ``ww_split``: parts a water group's union is cut into (more parts shorten
+  the last wave, each repeats the per-group set-up);
 * ``spme_grid``: the SPME grid among FFT-friendly sizes whose spacing is at
   most the configured grid's (the accuracy rule: a finer grid is never less
   accurate, so every candidate holds the force tolerance), at the
@@ -151,7 +150,7 @@ def tune(system, cfg, steps=100, warmup=20, tie=0.02, cache=True, stream=None, l
             return dict(hit)
     cur = {"neighbor_skin": float(cfg.neighbor_skin), "prune_buffer": float(cfg.prune_buffer or 0.4),
            "ww_union_chunk": int(cfg.ww_union_chunk), "ww_split": int(cfg.ww_split),
-           "pair_item_entries": int(cfg.pair_item_entries or 8),
+           "pair_item_entries": int(cfg.pair_item_entries or 4),
            "spme_grid_step": 0}
     has_water = len(np.asarray(system.get("water_pos", np.zeros((0, 3, 3))))) > 0
     has_atoms = len(np.asarray(system.get("atom_pos", np.zeros((0, 3))))) > 0

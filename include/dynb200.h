@@ -319,8 +319,8 @@ typedef struct {
                              * gather) takes them; 0 = about twice the mean.
                              * Results do not depend on it (integer sums). */
     uint32_t pair_item_entries; /* list entries per work item of the
-                             * water-atom and atom-atom pair kernels (1..32);
-                             * 0 = 8.  A tuning knob: results change only at
+                             * atom-atom pair kernel (1..32); 0 = automatic
+                             * (4).  A tuning knob: results change only at
                              * rounding level.                              */
     uint32_t ww_split;      /* CTAs that share one 32-water group's list
                              * entries in the water-water kernel (1..8);
