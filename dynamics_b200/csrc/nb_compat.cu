@@ -39,9 +39,17 @@ struct dyn_nb_s {
     float rc = 10.f, alpha = 0.3f, ljc = 0.f;
     float* d_pos[5] = {};          // dyn, O, M, H0, H1: [3n] floats
     long long* d_f[5] = {};        // fixed-point forces [3n]
-    double* d_partials = nullptr;  // [NB_MAX_BLOCKS * NB_PART]
+    double* d_partials = nullptr;  // [2 * NB_MAX_BLOCKS * NB_PART]
     double* d_scalars = nullptr;   // virial, energy, dH/dlambda
     uint64_t n_alch = 0;           // installed pairs with the alchemical bit
+    // device memory of dyn_nb_build_pairs, kept between calls: its inputs and
+    // row counts, and the lists of (row, neighbour) pairs
+    struct Area { char* p = nullptr; size_t cap = 0; };
+    Area scratch, lists;
+    // the installed list ends in the ten flat entries of each of these water
+    // pairs (in lists): every built list, and a set one in the same order
+    uint64_t n_ww = 0;
+    const uint32_t* d_wwi = nullptr; const uint32_t* d_wwj = nullptr;
     uint64_t n_pairs = 0, cap_pairs = 0;
     uint2* d_pidx = nullptr;       // packed target/source words
     float2* d_plj = nullptr;       // sigma, eps
@@ -120,99 +128,210 @@ __device__ __forceinline__ void soft_core(float r2, float sig, float eps, float 
 //   r <= lj_cutoff, energy when either body is an atom.
 // ALCH: pairs with the alchemical bit take soft-core LJ at the schedule's LJ
 //   lambda and Coulomb times its scale; their dH/dlambda is summed.
+struct PairConsts {
+    float3 ext, inv_ext;
+    float3 half;   // displacements below it are their own nearest image
+    float rc, alpha, ljc;
+    uint32_t ovr;
+};
+
+template <bool CPU_SEM>
+__device__ __forceinline__ float image1(float d, float ext, float inv_ext, float half) {
+    // |d| < half = 0.4999 extents: the quotient rounds to zero and d stays
+    if (fabsf(d) < half) return d;
+    if (CPU_SEM) return __fsub_rn(d, __fmul_rn(round_half_away(__fdiv_rn(d, ext)), ext));
+    return d - rintf(d * inv_ext) * ext;
+}
+
+// One pair with displacement d (nearest image) and r2 = |d|^2: its force on
+// the target is d times the returned value; e and dh receive its energy and
+// dH/dlambda.
+template <bool CPU_SEM, bool ALCH>
+__device__ __forceinline__ float pair_eval(float r2, float sigma, float eps, float qq, bool scale14, bool alch,
+                                           const PairConsts& c, const AlchSched& al, float& e, float& dh) {
+    e = 0.f;
+    dh = 0.f;
+    const bool lj_off = c.ovr & DYN_OVR_LJ_DISABLED;
+    const bool co_off = c.ovr & DYN_OVR_COULOMB_DISABLED;
+    if (r2 < (CPU_SEM ? 1e-12f : 1e-16f)) {
+        if (CPU_SEM && ALCH && alch && !lj_off && eps != 0.f) {
+            float fs;
+            soft_core(0.f, sigma, eps, al.ll, fs, e, dh);
+            if (scale14) { e *= 0.5f; dh *= 0.5f; }
+            dh *= al.dll;
+        }
+        return 0.f;
+    }
+    const float inv_r = rsqrtf(r2);
+    const float r = r2 * inv_r;
+    float fmag = 0.f;
+    if (!lj_off && eps != 0.f && (!CPU_SEM || r <= c.ljc)) {
+        float fl, el;
+        if (ALCH && alch) {
+            soft_core(r2, sigma, eps, al.ll, fl, el, dh);
+            dh *= al.dll;
+        } else {
+            const float sr = sigma * inv_r;
+            const float sr2 = sr * sr;
+            const float sr6 = sr2 * sr2 * sr2;
+            const float sr12 = sr6 * sr6;
+            fl = 24.0f * eps * fmaf(2.f, sr12, -sr6) * inv_r;
+            el = 4.f * eps * (sr12 - sr6);
+        }
+        if (scale14) { fl *= 0.5f; el *= 0.5f; dh *= 0.5f; }
+        fmag += fl; e += el;
+    }
+    if (!co_off && qq != 0.f && r < c.rc) {
+        const float ar = c.alpha * r;
+        const float ec = erfcf(ar);
+        const float ex = expf(-(ar * ar));
+        float fc = qq * fmaf(ec, inv_r * inv_r, 2.0f * c.alpha * ex * INV_SQRT_PI_F * inv_r);
+        float eco = qq * inv_r * ec;
+        if (scale14) { fc *= 0.833333333f; eco *= 0.833333333f; }
+        if (ALCH && alch) {
+            fmag += fc * al.cs; e += eco * al.cs;
+            dh += eco * al.dcs;
+        } else {
+            fmag += fc; e += eco;
+        }
+    }
+    return fmag * inv_r;
+}
+
+__device__ __forceinline__ void write_nb_partials(double w, double e, double h, double* __restrict__ partials) {
+    double v[NB_PART] = {w, e, h};
+    block_sum_d<NB_PART>(v);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < NB_PART; ++k) partials[NB_PART * blockIdx.x + k] = v[k];
+}
+
+__device__ __forceinline__ double virial_of(float3 d, float3 f) {
+    return (double)d.x * (double)f.x + (double)d.y * (double)f.y + (double)d.z * (double)f.z;
+}
+
+// The general kernel: any flat pair list, one pair per thread.  Pairs beyond
+// the cutoffs (most of a list with the reference's 4 A skin) add nothing and
+// skip their six 64-bit reductions, which bound the kernel.
 template <bool CPU_SEM, bool ALCH>
 __global__ void __launch_bounds__(NB_BLOCK) nb_pair_kernel(
     PosPtrs pos, ForcePtrs out, const uint2* __restrict__ pidx, const float2* __restrict__ plj,
-    const float* __restrict__ pqq, uint64_t n, float3 ext, float3 inv_ext, float rc, float alpha,
-    float ljc, uint32_t ovr, AlchSched al, double* __restrict__ partials) {
+    const float* __restrict__ pqq, uint64_t n, PairConsts c, AlchSched al, double* __restrict__ partials) {
     double w_acc = 0.0, e_acc = 0.0, h_acc = 0.0;
-    const bool lj_off = ovr & DYN_OVR_LJ_DISABLED;
-    const bool co_off = ovr & DYN_OVR_COULOMB_DISABLED;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
          p += (uint64_t)gridDim.x * blockDim.x) {
         const uint2 w = pidx[p];
         const uint32_t bt = (w.x >> 28) & 7u, bs = (w.y >> 28) & 7u;
         const uint32_t it = w.x & TGT_MASK, is = w.y & IDX_MASK;
         const bool scale14 = w.x >> 31, sym = w.y >> 31;
-        const bool alch = ALCH && (w.x & ALCH_BIT);
-        const bool e_counts = CPU_SEM ? (bt == 0 || bs == 0) : (bt == 0);
         const float3 pt = ld_pos(pos.p, bt, it);
         const float3 ps = ld_pos(pos.p, bs, is);
         float3 d = pt - ps;
-        if (CPU_SEM) {
-            d.x = __fsub_rn(d.x, __fmul_rn(round_half_away(__fdiv_rn(d.x, ext.x)), ext.x));
-            d.y = __fsub_rn(d.y, __fmul_rn(round_half_away(__fdiv_rn(d.y, ext.y)), ext.y));
-            d.z = __fsub_rn(d.z, __fmul_rn(round_half_away(__fdiv_rn(d.z, ext.z)), ext.z));
-        } else {
-            d.x -= rintf(d.x * inv_ext.x) * ext.x;
-            d.y -= rintf(d.y * inv_ext.y) * ext.y;
-            d.z -= rintf(d.z * inv_ext.z) * ext.z;
-        }
+        d.x = image1<CPU_SEM>(d.x, c.ext.x, c.inv_ext.x, c.half.x);
+        d.y = image1<CPU_SEM>(d.y, c.ext.y, c.inv_ext.y, c.half.y);
+        d.z = image1<CPU_SEM>(d.z, c.ext.z, c.inv_ext.z, c.half.z);
         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
         const float2 lj = plj[p];
-        if (r2 < (CPU_SEM ? 1e-12f : 1e-16f)) {
-            if (CPU_SEM && alch && !lj_off && lj.y != 0.f) {
-                float fs, es, dv;
-                soft_core(0.f, lj.x, lj.y, al.ll, fs, es, dv);
-                if (scale14) { es *= 0.5f; dv *= 0.5f; }
-                if (e_counts) e_acc += (double)es;
-                h_acc += (double)(dv * al.dll);
-            }
-            continue;
-        }
-        const float inv_r = rsqrtf(r2);
-        const float r = r2 * inv_r;
-        float fmag = 0.f, e = 0.f, dh = 0.f;
-        if (!lj_off && lj.y != 0.f && (!CPU_SEM || r <= ljc)) {
-            float fl, el;
-            if (alch) {
-                soft_core(r2, lj.x, lj.y, al.ll, fl, el, dh);
-                dh *= al.dll;
-            } else {
-                const float sr = lj.x * inv_r;
-                const float sr2 = sr * sr;
-                const float sr6 = sr2 * sr2 * sr2;
-                const float sr12 = sr6 * sr6;
-                fl = 24.0f * lj.y * fmaf(2.f, sr12, -sr6) * inv_r;
-                el = 4.f * lj.y * (sr12 - sr6);
-            }
-            if (scale14) { fl *= 0.5f; el *= 0.5f; dh *= 0.5f; }
-            fmag += fl; e += el;
-        }
-        const float qq = pqq[p];
-        if (!co_off && qq != 0.f && r < rc) {
-            const float ar = alpha * r;
-            const float ec = erfcf(ar);
-            const float ex = expf(-(ar * ar));
-            float fc = qq * fmaf(ec, inv_r * inv_r, 2.0f * alpha * ex * INV_SQRT_PI_F * inv_r);
-            float eco = qq * inv_r * ec;
-            if (scale14) { fc *= 0.833333333f; eco *= 0.833333333f; }
-            if (alch) {
-                fmag += fc * al.cs; e += eco * al.cs;
-                dh += eco * al.dcs;
-            } else {
-                fmag += fc; e += eco;
-            }
-        }
-        const float3 f = d * (fmag * inv_r);
-        w_acc += (double)d.x * (double)f.x + (double)d.y * (double)f.y + (double)d.z * (double)f.z;
-        if (e_counts) e_acc += (double)e;
+        float e, dh;
+        const float fs = pair_eval<CPU_SEM, ALCH>(r2, lj.x, lj.y, pqq[p], scale14, ALCH && (w.x & ALCH_BIT), c, al, e, dh);
+        if (CPU_SEM ? (bt == 0 || bs == 0) : (bt == 0)) e_acc += (double)e;
         if (ALCH) h_acc += (double)dh;
+        if (fs == 0.f && isfinite(r2)) continue;
+        const float3 f = d * fs;
+        w_acc += virial_of(d, f);
         long long* ft = out.f[bt] + 3 * (size_t)it;
         fix_atomic_add(ft + 0, fix_from_float(f.x));
         fix_atomic_add(ft + 1, fix_from_float(f.y));
         fix_atomic_add(ft + 2, fix_from_float(f.z));
         if (sym) {
-            long long* fs = out.f[bs] + 3 * (size_t)is;
-            fix_atomic_add(fs + 0, -fix_from_float(f.x));
-            fix_atomic_add(fs + 1, -fix_from_float(f.y));
-            fix_atomic_add(fs + 2, -fix_from_float(f.z));
+            long long* fsrc = out.f[bs] + 3 * (size_t)is;
+            fix_atomic_add(fsrc + 0, -fix_from_float(f.x));
+            fix_atomic_add(fsrc + 1, -fix_from_float(f.y));
+            fix_atomic_add(fsrc + 2, -fix_from_float(f.z));
         }
     }
-    double v[NB_PART] = {w_acc, e_acc, h_acc};
-    block_sum_d<NB_PART>(v);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < NB_PART; ++k) partials[NB_PART * blockIdx.x + k] = v[k];
+    write_nb_partials(w_acc, e_acc, h_acc, partials);
+}
+
+// The water-water part of a list in setup_pairs' order, from its
+// molecule pairs (8 bytes each) instead of their ten flat entries (200 bytes).
+// A thread takes run consecutive molecule pairs, which mostly share the
+// first water: every site pair is evaluated and rounded to fixed point as by
+// the general kernel, the first water's forces are summed in 64-bit registers
+// until it changes and the second's per molecule pair, so the sums are the
+// same integers.  Bound by issue (pairs beyond the cutoff cost their distance
+// only).  1.4 M molecule pairs of 7,800 waters (13 A list, 9 A cutoff): 148 us,
+// against 942 us for their 14 M flat entries with six reductions each.  Runs
+// of 8 where that leaves four waves of threads, shorter ones below (89,000
+// molecule pairs in runs of 8 left most of the SMs without work: 58 us).
+constexpr uint64_t WW_RUN = 8, WW_THREADS = 148 * 1024;
+inline uint32_t ww_run(uint64_t n) { return (uint32_t)std::max<uint64_t>(1, std::min(WW_RUN, n / WW_THREADS)); }
+
+template <bool CPU_SEM>
+__global__ void __launch_bounds__(NB_BLOCK) nb_ww_kernel(PosPtrs pos, ForcePtrs out, const uint32_t* __restrict__ wi,
+                                                         const uint32_t* __restrict__ wj, uint64_t n, uint32_t run,
+                                                         PairConsts c, double* __restrict__ partials) {
+    // sites in setup_pairs' order O, M, H0, H1 = bodies 1..4
+    const float q[4] = {0.f, OPC_Q_EP, OPC_Q_H, OPC_Q_H};
+    const AlchSched none{1.f, 0.f, 0.f, 0.f};
+    double w_acc = 0.0;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * run;
+    for (uint64_t k0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * run; k0 < n; k0 += stride) {
+        const uint64_t k1 = k0 + run < n ? k0 + run : n;
+        uint32_t cur = 0xFFFFFFFFu;
+        float3 pi[4];
+        long long fi[12];
+        bool any_i = false;
+        auto flush = [&]() {
+            if (any_i)
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+                        if (fi[3 * s + x]) fix_atomic_add(out.f[s + 1] + 3 * (size_t)cur + x, fi[3 * s + x]);
+        };
+        for (uint64_t k = k0; k < k1; ++k) {
+            const uint32_t i = wi[k], j = wj[k];
+            if (i != cur) {
+                flush();
+                cur = i;
+                any_i = false;
+#pragma unroll
+                for (int s = 0; s < 4; ++s) pi[s] = ld_pos(pos.p, s + 1, i);
+#pragma unroll
+                for (int x = 0; x < 12; ++x) fi[x] = 0;
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float3 pj = ld_pos(pos.p, t + 1, j);
+                long long fj[3] = {0, 0, 0};
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    if ((s == 0) != (t == 0)) continue;  // O-O (LJ) and the charged sites' pairs
+                    float3 d = pi[s] - pj;
+                    d.x = image1<CPU_SEM>(d.x, c.ext.x, c.inv_ext.x, c.half.x);
+                    d.y = image1<CPU_SEM>(d.y, c.ext.y, c.inv_ext.y, c.half.y);
+                    d.z = image1<CPU_SEM>(d.z, c.ext.z, c.inv_ext.z, c.half.z);
+                    const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+                    float e, dh;
+                    const float fs = pair_eval<CPU_SEM, false>(r2, OPC_O_SIGMA, s == 0 ? OPC_O_EPS : 0.f,
+                                                               s == 0 ? 0.f : __fmul_rn(q[s], q[t]), false, false, c,
+                                                               none, e, dh);
+                    if (fs == 0.f && isfinite(r2)) continue;
+                    const float3 f = d * fs;
+                    w_acc += virial_of(d, f);
+                    const long long x = fix_from_float(f.x), y = fix_from_float(f.y), z = fix_from_float(f.z);
+                    fi[3 * s + 0] += x; fi[3 * s + 1] += y; fi[3 * s + 2] += z;
+                    fj[0] -= x; fj[1] -= y; fj[2] -= z;
+                    any_i = true;
+                }
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                    if (fj[x]) fix_atomic_add(out.f[t + 1] + 3 * (size_t)j + x, fj[x]);
+            }
+        }
+        flush();
+    }
+    write_nb_partials(w_acc, 0.0, 0.0, partials);
 }
 
 // Sums block partials in a fixed order (deterministic).
@@ -327,8 +446,8 @@ struct ListArgs {
 // PASS 0 counts pairs per row; PASS 1 writes them at row offsets.
 template <int PASS>
 __global__ void ref_list_kernel(ListArgs a, uint32_t* __restrict__ row_count,
-                                const uint64_t* __restrict__ row_off, uint32_t* __restrict__ out_j,
-                                uint8_t* __restrict__ out_s14) {
+                                const uint64_t* __restrict__ row_off, uint32_t* __restrict__ out_i,
+                                uint32_t* __restrict__ out_j, uint8_t* __restrict__ out_s14) {
     const int lane = threadIdx.x & 31;
     const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= a.n_outer) return;
@@ -360,6 +479,7 @@ __global__ void ref_list_kernel(ListArgs a, uint32_t* __restrict__ row_count,
         const uint32_t m = __ballot_sync(0xffffffffu, hit);
         if (PASS && hit) {
             const uint32_t k = cnt + __popc(m & ((1u << lane) - 1u));
+            out_i[base + k] = row;
             out_j[base + k] = j;
             if (out_s14) out_s14[base + k] = s14;
         }
@@ -368,13 +488,53 @@ __global__ void ref_list_kernel(ListArgs a, uint32_t* __restrict__ row_count,
     if (!PASS && lane == 0) row_count[row] = cnt;
 }
 
-// Emits the flat SoA of setup_pairs from the per-row neighbour arrays.
+// Exclusive sums of the rows' counts and their total, a block per list.
+struct ScanArgs { const uint32_t* cnt[3]; uint64_t* off[3]; uint32_t n[3]; uint64_t* total; };
+constexpr int SCAN_T = 1024;
+__global__ void __launch_bounds__(SCAN_T) scan_rows_kernel(ScanArgs a) {
+    __shared__ uint64_t ws[SCAN_T / 32];
+    const uint32_t* cnt = a.cnt[blockIdx.x];
+    uint64_t* off = a.off[blockIdx.x];
+    const uint32_t n = a.n[blockIdx.x];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint64_t base = 0;
+    for (uint64_t c0 = 0; c0 < n; c0 += SCAN_T) {
+        const uint64_t c = c0 + threadIdx.x;
+        const uint64_t k = c < n ? cnt[c] : 0u;
+        uint64_t x = k;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[w] = x;
+        __syncthreads();
+        if (w == 0) {
+            uint64_t t = ws[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t y = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= o) t += y;
+            }
+            ws[lane] = t;
+        }
+        __syncthreads();
+        if (c < n) off[c] = base + (w ? ws[w - 1] : 0u) + x - k;
+        base += ws[SCAN_T / 32 - 1];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) { off[n] = base; a.total[blockIdx.x] = base; }
+}
+
+// The flat SoA of setup_pairs from the three lists of (row, neighbour)
+// pairs, one flat entry per thread so that the writes are contiguous: 0.9 M
+// entries in 5 us; a thread per row, whose lanes wrote 200 bytes apart, took
+// 698 us for the water part and 260 for the water-atom part.
 struct EmitArgs {
-    uint32_t n_std, n_water;
-    const uint64_t* ss_off; const uint32_t* ss_j; const uint8_t* ss_s14;
-    const uint64_t* sw_off; const uint32_t* sw_j;
-    const uint64_t* ww_off; const uint32_t* ww_j;
-    uint64_t base_sw, base_ww;
+    uint64_t n_ss, n_sw, n_ww;  // list entries
+    const uint32_t* ss_i; const uint32_t* ss_j; const uint8_t* ss_s14;
+    const uint32_t* sw_i; const uint32_t* sw_j;
+    const uint32_t* ww_i; const uint32_t* ww_j;
     const float* q; const float* sig; const float* eps;
 };
 
@@ -383,55 +543,41 @@ __device__ __forceinline__ float site_q(uint32_t s) {
     return s == DYN_BODY_W_O ? 0.f : (s == DYN_BODY_W_M ? OPC_Q_EP : OPC_Q_H);
 }
 
-__global__ void emit_ss_kernel(EmitArgs a, uint2* pidx, float2* plj, float* pqq) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n_std) return;
-    for (uint64_t k = a.ss_off[i]; k < a.ss_off[i + 1]; ++k) {
-        const uint32_t j = a.ss_j[k];
-        const bool s14 = a.ss_s14[k];
-        pidx[k] = make_uint2(i | (s14 ? 0x80000000u : 0u), j | 0x80000000u);
-        // combine_lj_params (src/non_bonded.rs:1081-1086)
-        plj[k] = make_float2(__fmul_rn(0.5f, __fadd_rn(a.sig[i], a.sig[j])),
-                             __fsqrt_rn(__fmul_rn(a.eps[i], a.eps[j])));
-        pqq[k] = __fmul_rn(a.q[i], a.q[j]);
-    }
-}
-
-__global__ void emit_sw_kernel(EmitArgs a, uint2* pidx, float2* plj, float* pqq) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n_std) return;
-    // water_std row of LjTables (src/non_bonded.rs:139-145)
-    const float sg = __fmul_rn(0.5f, __fadd_rn(a.sig[i], OPC_O_SIGMA));
-    const float ep = __fsqrt_rn(__fmul_rn(a.eps[i], OPC_O_EPS));
-    for (uint64_t k = a.sw_off[i]; k < a.sw_off[i + 1]; ++k) {
-        const uint32_t w = a.sw_j[k];
-        const uint64_t o = a.base_sw + 4 * k;
-        const uint32_t sites[4] = {DYN_BODY_W_O, DYN_BODY_W_M, DYN_BODY_W_H0, DYN_BODY_W_H1};
-        for (int s = 0; s < 4; ++s) {
-            pidx[o + s] = make_uint2(i, w | (sites[s] << 28) | 0x80000000u);
-            plj[o + s] = make_float2(sg, s == 0 ? ep : 0.f);
-            pqq[o + s] = s == 0 ? 0.f : __fmul_rn(a.q[i], site_q(sites[s]));
+__global__ void __launch_bounds__(NB_BLOCK) emit_pairs_kernel(EmitArgs a, uint2* __restrict__ pidx,
+                                                              float2* __restrict__ plj, float* __restrict__ pqq) {
+    const uint64_t base_sw = a.n_ss, base_ww = base_sw + 4 * a.n_sw, n = base_ww + 10 * a.n_ww;
+    for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < n; o += (uint64_t)gridDim.x * blockDim.x) {
+        uint2 w;
+        float2 lj;
+        float qq;
+        if (o >= base_ww) {
+            // O-O, then M, H0, H1 against M, H0, H1
+            const uint64_t k = (o - base_ww) / 10u;
+            const uint32_t t = (uint32_t)((o - base_ww) - 10u * k);
+            const uint32_t s0 = t ? DYN_BODY_W_M + (t - 1) / 3u : DYN_BODY_W_O;
+            const uint32_t s1 = t ? DYN_BODY_W_M + (t - 1) % 3u : DYN_BODY_W_O;
+            w = make_uint2(a.ww_i[k] | (s0 << 28), a.ww_j[k] | (s1 << 28) | 0x80000000u);
+            lj = make_float2(OPC_O_SIGMA, t ? 0.f : OPC_O_EPS);
+            qq = t ? __fmul_rn(site_q(s0), site_q(s1)) : 0.f;
+        } else if (o >= base_sw) {
+            const uint64_t k = (o - base_sw) >> 2;
+            const uint32_t s = DYN_BODY_W_O + (uint32_t)((o - base_sw) & 3u);
+            const uint32_t i = a.sw_i[k];
+            w = make_uint2(i, a.sw_j[k] | (s << 28) | 0x80000000u);
+            // water_std row of LjTables (src/non_bonded.rs:139-145)
+            lj = make_float2(__fmul_rn(0.5f, __fadd_rn(a.sig[i], OPC_O_SIGMA)),
+                             s == DYN_BODY_W_O ? __fsqrt_rn(__fmul_rn(a.eps[i], OPC_O_EPS)) : 0.f);
+            qq = s == DYN_BODY_W_O ? 0.f : __fmul_rn(a.q[i], site_q(s));
+        } else {
+            const uint32_t i = a.ss_i[o], j = a.ss_j[o];
+            w = make_uint2(i | (a.ss_s14[o] ? 0x80000000u : 0u), j | 0x80000000u);
+            // combine_lj_params (src/non_bonded.rs:1081-1086)
+            lj = make_float2(__fmul_rn(0.5f, __fadd_rn(a.sig[i], a.sig[j])), __fsqrt_rn(__fmul_rn(a.eps[i], a.eps[j])));
+            qq = __fmul_rn(a.q[i], a.q[j]);
         }
-    }
-}
-
-__global__ void emit_ww_kernel(EmitArgs a, uint2* pidx, float2* plj, float* pqq) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n_water) return;
-    const uint32_t sites[4] = {DYN_BODY_W_O, DYN_BODY_W_M, DYN_BODY_W_H0, DYN_BODY_W_H1};
-    for (uint64_t k = a.ww_off[i]; k < a.ww_off[i + 1]; ++k) {
-        const uint32_t j = a.ww_j[k];
-        uint64_t o = a.base_ww + 10 * k;
-        for (int s0 = 0; s0 < 4; ++s0)
-            for (int s1 = 0; s1 < 4; ++s1) {
-                const bool lj = s0 == 0 && s1 == 0;
-                const bool co = s0 != 0 && s1 != 0;
-                if (!(lj || co)) continue;
-                pidx[o] = make_uint2(i | (sites[s0] << 28), j | (sites[s1] << 28) | 0x80000000u);
-                plj[o] = make_float2(OPC_O_SIGMA, lj ? OPC_O_EPS : 0.f);
-                pqq[o] = co ? __fmul_rn(site_q(sites[s0]), site_q(sites[s1])) : 0.f;
-                ++o;
-            }
+        pidx[o] = w;
+        plj[o] = lj;
+        pqq[o] = qq;
     }
 }
 
@@ -484,18 +630,44 @@ void build_csr(uint32_t n, uint64_t m, const uint32_t* pairs, std::vector<uint32
     }
 }
 
-// exclusive scan of row counts on the host (rows are few relative to pairs)
-int scan_rows(cudaStream_t st, const uint32_t* d_cnt, uint32_t n, uint64_t* d_off,
-              uint64_t* total) {
-    std::vector<uint32_t> c(n);
-    std::vector<uint64_t> o(n + 1, 0);
-    if (n) DYN_CUDA(cudaMemcpyAsync(c.data(), d_cnt, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    DYN_CUDA(cudaStreamSynchronize(st));
-    for (uint32_t i = 0; i < n; ++i) o[i + 1] = o[i] + c[i];
-    DYN_CUDA(cudaMemcpyAsync(d_off, o.data(), (n + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    DYN_CUDA(cudaStreamSynchronize(st));
-    *total = o[n];
+// Whether the ten entries from o on are one water pair as setup_pairs writes
+// it (emit_pairs_kernel): O-O with the water's LJ, then M, H0, H1 against M,
+// H0, H1 with their charges, all symmetric.
+bool is_water_pair(uint64_t o, const uint32_t* tgt, const uint32_t* src, const float* sigma, const float* eps,
+                   const float* q_tgt, const float* q_src, const uint8_t* body_tgt, const uint8_t* body_src,
+                   const uint8_t* flags) {
+    const float q[3] = {OPC_Q_EP, OPC_Q_H, OPC_Q_H};
+    for (uint32_t t = 0; t < 10; ++t) {
+        const uint64_t p = o + t;
+        const uint32_t s0 = t ? (t - 1) / 3u : 0u, s1 = t ? (t - 1) % 3u : 0u;
+        if (tgt[p] != tgt[o] || src[p] != src[o] || body_tgt[p] != (t ? DYN_BODY_W_M + s0 : DYN_BODY_W_O) ||
+            body_src[p] != (t ? DYN_BODY_W_M + s1 : DYN_BODY_W_O) ||
+            flags[p] != (DYN_PAIR_SYMMETRIC | (t ? DYN_PAIR_COULOMB : DYN_PAIR_LJ)))
+            return false;
+        if (t ? q_tgt[p] * q_src[p] != q[s0] * q[s1] : sigma[p] != OPC_O_SIGMA || eps[p] != OPC_O_EPS) return false;
+    }
+    return true;
+}
+
+// Device memory of a handle that grows as calls need more and is kept.
+int ensure(dyn_nb_s::Area& a, size_t bytes) {
+    if (bytes <= a.cap) return DYN_OK;
+    if (a.p) cudaFree(a.p);
+    a.p = nullptr;
+    a.cap = 0;
+    const cudaError_t e = cudaMalloc((void**)&a.p, bytes);
+    if (e != cudaSuccess) return dyn::cuda_fail(e, "cudaMalloc");
+    a.cap = bytes;
     return DYN_OK;
+}
+
+// Takes n elements from an area laid out front to back (256-byte aligned);
+// with base = nullptr only the size is counted.
+template <typename T>
+T* carve(char* base, size_t& used, size_t n) {
+    T* p = base ? (T*)(base + used) : nullptr;
+    used += (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+    return p;
 }
 
 }  // namespace
@@ -519,7 +691,7 @@ extern "C" int dyn_nb_create(void* stream, uint32_t n_dyn, uint32_t n_water, flo
             (rc = halloc(&h->h_pos[a], n3)) || (rc = halloc(&h->h_f[a], n3)))
             break;
     }
-    if (rc == DYN_OK) rc = dalloc(&h->d_partials, NB_PART * NB_MAX_BLOCKS);
+    if (rc == DYN_OK) rc = dalloc(&h->d_partials, 2 * NB_PART * NB_MAX_BLOCKS);
     if (rc == DYN_OK) rc = dalloc(&h->d_scalars, NB_PART);
     if (rc == DYN_OK) rc = halloc(&h->h_scalars, NB_PART);
     if (rc != DYN_OK) {
@@ -539,6 +711,7 @@ extern "C" int dyn_nb_destroy(dyn_nb_t h) {
     }
     cudaFree(h->d_partials); cudaFree(h->d_scalars); cudaFreeHost(h->h_scalars);
     cudaFree(h->d_pidx); cudaFree(h->d_plj); cudaFree(h->d_pqq);
+    cudaFree(h->scratch.p); cudaFree(h->lists.p);
     delete h;
     return DYN_OK;
 }
@@ -561,6 +734,7 @@ extern "C" int dyn_nb_set_pairs(dyn_nb_t h, uint64_t n, const uint32_t* tgt, con
     if (rc) return rc;
     h->n_pairs = n;
     h->n_alch = 0;
+    h->n_ww = 0;
     for (uint64_t p = 0; p < n; ++p) h->n_alch += (flags[p] & DYN_PAIR_ALCH) != 0;
     if (n == 0) return DYN_OK;
     // stage through temporary device buffers, then pack
@@ -593,6 +767,35 @@ extern "C" int dyn_nb_set_pairs(dyn_nb_t h, uint64_t n, const uint32_t* tgt, con
     DYN_CUDA(cudaGetLastError());
     DYN_CUDA(cudaStreamSynchronize(st));
     cudaFree(tmp);
+    // the water pairs a list in setup_pairs' order ends with are evaluated by
+    // molecule, as those of a built list
+    uint64_t nww = 0;
+    while (10 * (nww + 1) <= n &&
+           is_water_pair(n - 10 * (nww + 1), tgt, src, sigma, eps, q_tgt, q_src, body_tgt, body_src, flags))
+        ++nww;
+    if (nww) {
+        std::vector<uint32_t> wi(nww), wj(nww);
+        for (uint64_t k = 0; k < nww; ++k) {
+            const uint64_t o = n - 10 * (nww - k);
+            wi[k] = tgt[o];
+            wj[k] = src[o];
+        }
+        uint32_t *di = nullptr, *dj = nullptr;
+        auto lay = [&](char* base) {
+            size_t u = 0;
+            di = carve<uint32_t>(base, u, nww);
+            dj = carve<uint32_t>(base, u, nww);
+            return u;
+        };
+        if ((rc = ensure(h->lists, lay(nullptr))) != DYN_OK) return rc;
+        lay(h->lists.p);
+        DYN_CUDA(cudaMemcpyAsync(di, wi.data(), 4 * nww, cudaMemcpyHostToDevice, st));
+        DYN_CUDA(cudaMemcpyAsync(dj, wj.data(), 4 * nww, cudaMemcpyHostToDevice, st));
+        DYN_CUDA(cudaStreamSynchronize(st));
+        h->d_wwi = di;
+        h->d_wwj = dj;
+        h->n_ww = nww;
+    }
     return DYN_OK;
 }
 
@@ -664,94 +867,121 @@ extern "C" int dyn_nb_build_pairs(dyn_nb_t h, const float* pos_dyn, const float*
     std::vector<uint32_t> ex_off, ex_idx, s_off, s_idx;
     build_csr(ns, n_excl, excl, ex_off, ex_idx);
     build_csr(ns, n_pair14, pair14, s_off, s_idx);
-    // device scratch
-    float *d_atoms = nullptr, *d_wo = nullptr, *d_wo_raw = nullptr, *d_q = nullptr, *d_sig = nullptr,
-          *d_eps = nullptr;
-    uint8_t *d_static = nullptr, *d_bonly = nullptr, *d_s14 = nullptr;
-    uint32_t *d_exo = nullptr, *d_exi = nullptr, *d_so = nullptr, *d_si = nullptr, *d_cnt = nullptr,
-             *d_ssj = nullptr, *d_swj = nullptr, *d_wwj = nullptr;
-    uint64_t *d_sso = nullptr, *d_swo = nullptr, *d_wwo = nullptr;
-    int rc = DYN_OK;
-    auto cleanup = [&]() {
-        cudaFree(d_atoms); cudaFree(d_wo); cudaFree(d_wo_raw); cudaFree(d_q); cudaFree(d_sig);
-        cudaFree(d_eps); cudaFree(d_static); cudaFree(d_bonly); cudaFree(d_s14); cudaFree(d_exo);
-        cudaFree(d_exi); cudaFree(d_so); cudaFree(d_si); cudaFree(d_cnt); cudaFree(d_ssj);
-        cudaFree(d_swj); cudaFree(d_wwj); cudaFree(d_sso); cudaFree(d_swo); cudaFree(d_wwo);
+#define TRY(x) do { const int _r = (x); if (_r != DYN_OK) return _r; } while (0)
+    // the inputs, packed on the host and copied in one go, then the rows'
+    // counts and offsets
+    struct Lay {
+        float *atoms, *wo_raw, *q, *sig, *eps, *wo;
+        uint32_t *exo, *exi, *so, *si, *cnt[3];
+        uint8_t *st, *bonly;
+        uint64_t *off[3], *total;
+    } L{};
+    const uint32_t rows[3] = {ns, ns, nw};
+    auto lay = [&](char* base, size_t& in_bytes) {
+        size_t u = 0;
+        L.atoms = carve<float>(base, u, 3 * (size_t)ns);
+        L.wo_raw = carve<float>(base, u, 3 * (size_t)nw);
+        L.q = carve<float>(base, u, ns);
+        L.sig = carve<float>(base, u, ns);
+        L.eps = carve<float>(base, u, ns);
+        L.exo = carve<uint32_t>(base, u, ex_off.size());
+        L.exi = carve<uint32_t>(base, u, ex_idx.size());
+        L.so = carve<uint32_t>(base, u, s_off.size());
+        L.si = carve<uint32_t>(base, u, s_idx.size());
+        L.st = carve<uint8_t>(base, u, ns);
+        L.bonly = carve<uint8_t>(base, u, ns);
+        in_bytes = u;
+        L.wo = carve<float>(base, u, 3 * (size_t)nw);
+        for (int k = 0; k < 3; ++k) L.cnt[k] = carve<uint32_t>(base, u, rows[k]);
+        for (int k = 0; k < 3; ++k) L.off[k] = carve<uint64_t>(base, u, rows[k] + 1);
+        L.total = carve<uint64_t>(base, u, 3);
+        return u;
     };
-#define TRY(x) do { if ((rc = (x)) != DYN_OK) { cleanup(); return rc; } } while (0)
-#define TRYC(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { cleanup(); return dyn::cuda_fail(_e, #x); } } while (0)
-    TRY(dalloc(&d_atoms, 3 * (size_t)ns)); TRY(dalloc(&d_q, ns)); TRY(dalloc(&d_sig, ns));
-    TRY(dalloc(&d_eps, ns)); TRY(dalloc(&d_wo, 3 * (size_t)nw)); TRY(dalloc(&d_wo_raw, 3 * (size_t)nw));
-    TRY(dalloc(&d_exo, ns + 1)); TRY(dalloc(&d_exi, ex_idx.size())); TRY(dalloc(&d_so, ns + 1));
-    TRY(dalloc(&d_si, s_idx.size())); TRY(dalloc(&d_cnt, std::max(ns, nw)));
-    TRY(dalloc(&d_sso, ns + 1)); TRY(dalloc(&d_swo, ns + 1)); TRY(dalloc(&d_wwo, nw + 1));
-    if (is_static) { TRY(dalloc(&d_static, ns)); TRYC(cudaMemcpyAsync(d_static, is_static, ns, cudaMemcpyHostToDevice, st)); }
-    if (bonded_only) { TRY(dalloc(&d_bonly, ns)); TRYC(cudaMemcpyAsync(d_bonly, bonded_only, ns, cudaMemcpyHostToDevice, st)); }
-    if (ns) {
-        TRYC(cudaMemcpyAsync(d_atoms, pos_dyn, 12 * (size_t)ns, cudaMemcpyHostToDevice, st));
-        TRYC(cudaMemcpyAsync(d_q, atom_q, 4 * (size_t)ns, cudaMemcpyHostToDevice, st));
-        TRYC(cudaMemcpyAsync(d_sig, atom_sigma, 4 * (size_t)ns, cudaMemcpyHostToDevice, st));
-        TRYC(cudaMemcpyAsync(d_eps, atom_eps, 4 * (size_t)ns, cudaMemcpyHostToDevice, st));
-    }
-    TRYC(cudaMemcpyAsync(d_exo, ex_off.data(), 4 * ex_off.size(), cudaMemcpyHostToDevice, st));
-    if (!ex_idx.empty()) TRYC(cudaMemcpyAsync(d_exi, ex_idx.data(), 4 * ex_idx.size(), cudaMemcpyHostToDevice, st));
-    TRYC(cudaMemcpyAsync(d_so, s_off.data(), 4 * s_off.size(), cudaMemcpyHostToDevice, st));
-    if (!s_idx.empty()) TRYC(cudaMemcpyAsync(d_si, s_idx.data(), 4 * s_idx.size(), cudaMemcpyHostToDevice, st));
+    size_t in_bytes = 0;
+    TRY(ensure(h->scratch, lay(nullptr, in_bytes)));
+    std::vector<char> in(in_bytes);
+    lay(in.data(), in_bytes);
+    auto put = [](void* dst, const void* src, size_t n) { if (n && src) std::memcpy(dst, src, n); };
+    put(L.atoms, pos_dyn, 12 * (size_t)ns);
+    put(L.wo_raw, pos_w_o, 12 * (size_t)nw);
+    put(L.q, atom_q, 4 * (size_t)ns);
+    put(L.sig, atom_sigma, 4 * (size_t)ns);
+    put(L.eps, atom_eps, 4 * (size_t)ns);
+    put(L.exo, ex_off.data(), 4 * ex_off.size());
+    put(L.exi, ex_idx.data(), 4 * ex_idx.size());
+    put(L.so, s_off.data(), 4 * s_off.size());
+    put(L.si, s_idx.data(), 4 * s_idx.size());
+    put(L.st, is_static, ns);
+    put(L.bonly, bonded_only, ns);
+    lay(h->scratch.p, in_bytes);
+    DYN_CUDA(cudaMemcpyAsync(h->scratch.p, in.data(), in_bytes, cudaMemcpyHostToDevice, st));
     if (nw) {
-        TRYC(cudaMemcpyAsync(d_wo_raw, pos_w_o, 12 * (size_t)nw, cudaMemcpyHostToDevice, st));
-        wrap_o_kernel<<<(nw + 255) / 256, 256, 0, st>>>(nw, d_wo_raw, make_float3(lo_h[0], lo_h[1], lo_h[2]), ext, d_wo);
-        TRYC(cudaGetLastError());
+        wrap_o_kernel<<<(nw + 255) / 256, 256, 0, st>>>(nw, L.wo_raw, make_float3(lo_h[0], lo_h[1], lo_h[2]), ext, L.wo);
+        DYN_CUDA(cudaGetLastError());
     }
-    uint64_t n_ss = 0, n_sw = 0, n_ww = 0;
-    ListArgs la{};
-    la.thr = thr; la.ext = ext;
-    la.is_static = d_static; la.bonded_only = d_bonly;
-    la.ex_off = d_exo; la.ex_idx = d_exi; la.s14_off = d_so; la.s14_idx = d_si;
-    auto run_list = [&](const float* outer, const float* inner, uint32_t no, uint32_t ni, int mode,
-                        uint64_t* d_off, uint32_t** d_j, uint8_t** d_s14o, uint64_t* total) -> int {
-        ListArgs a = la;
-        a.outer = outer; a.inner = inner; a.n_outer = no; a.n_inner = ni; a.mode = mode;
-        if (mode != 0) { a.ex_off = nullptr; a.s14_off = nullptr; a.bonded_only = nullptr; a.is_static = nullptr; }
-        const int threads = 256;
-        const int blocks = (int)(((uint64_t)no * 32 + threads - 1) / threads);
-        if (no) {
-            ref_list_kernel<0><<<blocks, threads, 0, st>>>(a, d_cnt, nullptr, nullptr, nullptr);
-            DYN_CUDA(cudaGetLastError());
-        }
-        int r = scan_rows(st, d_cnt, no, d_off, total);
-        if (r) return r;
-        if ((r = dalloc(d_j, *total))) return r;
-        if (d_s14o && (r = dalloc(d_s14o, *total))) return r;
-        if (no) {
-            ref_list_kernel<1><<<blocks, threads, 0, st>>>(a, nullptr, d_off, *d_j, d_s14o ? *d_s14o : nullptr);
-            DYN_CUDA(cudaGetLastError());
-        }
-        return DYN_OK;
-    };
-    TRY(run_list(d_atoms, d_atoms, ns, ns, 0, d_sso, &d_ssj, &d_s14, &n_ss));
-    TRY(run_list(d_atoms, d_wo, ns, nw, 1, d_swo, &d_swj, nullptr, &n_sw));
-    TRY(run_list(d_wo, d_wo, nw, nw, 2, d_wwo, &d_wwj, nullptr, &n_ww));
-    const uint64_t total = n_ss + 4 * n_sw + 10 * n_ww;
-    TRY(ensure_pair_capacity(h, total));
-    EmitArgs ea{};
-    ea.n_std = ns; ea.n_water = nw;
-    ea.ss_off = d_sso; ea.ss_j = d_ssj; ea.ss_s14 = d_s14;
-    ea.sw_off = d_swo; ea.sw_j = d_swj; ea.ww_off = d_wwo; ea.ww_j = d_wwj;
-    ea.base_sw = n_ss; ea.base_ww = n_ss + 4 * n_sw;
-    ea.q = d_q; ea.sig = d_sig; ea.eps = d_eps;
-    if (ns) {
-        emit_ss_kernel<<<(ns + 127) / 128, 128, 0, st>>>(ea, h->d_pidx, h->d_plj, h->d_pqq);
-        emit_sw_kernel<<<(ns + 127) / 128, 128, 0, st>>>(ea, h->d_pidx, h->d_plj, h->d_pqq);
+    // std-std, std-water, water-water
+    ListArgs la[3];
+    for (int k = 0; k < 3; ++k) {
+        la[k] = ListArgs{};
+        la[k].thr = thr; la[k].ext = ext; la[k].mode = k;
+        la[k].outer = k == 2 ? L.wo : L.atoms;
+        la[k].inner = k == 0 ? L.atoms : L.wo;
+        la[k].n_outer = rows[k];
+        la[k].n_inner = k == 0 ? ns : nw;
     }
-    if (nw) emit_ww_kernel<<<(nw + 127) / 128, 128, 0, st>>>(ea, h->d_pidx, h->d_plj, h->d_pqq);
-    TRYC(cudaGetLastError());
-    TRYC(cudaStreamSynchronize(st));
-    h->n_pairs = total;
+    la[0].is_static = is_static ? L.st : nullptr;
+    la[0].bonded_only = bonded_only ? L.bonly : nullptr;
+    la[0].ex_off = L.exo; la[0].ex_idx = L.exi; la[0].s14_off = L.so; la[0].s14_idx = L.si;
+    const int threads = 256;
+    auto blocks = [&](int k) { return (unsigned)(((uint64_t)rows[k] * 32 + threads - 1) / threads); };
+    ScanArgs sa{};
+    for (int k = 0; k < 3; ++k) {
+        if (rows[k]) ref_list_kernel<0><<<blocks(k), threads, 0, st>>>(la[k], L.cnt[k], nullptr, nullptr, nullptr, nullptr);
+        sa.cnt[k] = L.cnt[k]; sa.off[k] = L.off[k]; sa.n[k] = rows[k];
+    }
+    sa.total = L.total;
+    scan_rows_kernel<<<3, SCAN_T, 0, st>>>(sa);
+    DYN_CUDA(cudaGetLastError());
+    uint64_t tot[3] = {};
+    DYN_CUDA(cudaMemcpyAsync(tot, L.total, sizeof(tot), cudaMemcpyDeviceToHost, st));
+    DYN_CUDA(cudaStreamSynchronize(st));
+    const uint64_t total = tot[0] + 4 * tot[1] + 10 * tot[2];
+    // nothing is installed while the list's memory is replaced
+    h->n_pairs = 0;
+    h->n_ww = 0;
     h->n_alch = 0;
+    uint32_t *li[3], *lj[3];
+    uint8_t* s14 = nullptr;
+    auto lay_lists = [&](char* base) {
+        size_t u = 0;
+        for (int k = 0; k < 3; ++k) { li[k] = carve<uint32_t>(base, u, tot[k]); lj[k] = carve<uint32_t>(base, u, tot[k]); }
+        s14 = carve<uint8_t>(base, u, tot[0]);
+        return u;
+    };
+    TRY(ensure(h->lists, lay_lists(nullptr)));
+    lay_lists(h->lists.p);
+    TRY(ensure_pair_capacity(h, total));
+    for (int k = 0; k < 3; ++k)
+        if (rows[k])
+            ref_list_kernel<1><<<blocks(k), threads, 0, st>>>(la[k], nullptr, L.off[k], li[k], lj[k], k == 0 ? s14 : nullptr);
+    EmitArgs ea{};
+    ea.n_ss = tot[0]; ea.n_sw = tot[1]; ea.n_ww = tot[2];
+    ea.ss_i = li[0]; ea.ss_j = lj[0]; ea.ss_s14 = s14;
+    ea.sw_i = li[1]; ea.sw_j = lj[1];
+    ea.ww_i = li[2]; ea.ww_j = lj[2];
+    ea.q = L.q; ea.sig = L.sig; ea.eps = L.eps;
+    if (total) {
+        const int eb = (int)std::min<uint64_t>((total + NB_BLOCK - 1) / NB_BLOCK, 148 * 16);
+        emit_pairs_kernel<<<eb, NB_BLOCK, 0, st>>>(ea, h->d_pidx, h->d_plj, h->d_pqq);
+    }
+    DYN_CUDA(cudaGetLastError());
+    DYN_CUDA(cudaStreamSynchronize(st));
+    h->n_pairs = total;
+    h->n_ww = tot[2];
+    h->d_wwi = li[2];
+    h->d_wwj = lj[2];
     if (n_pairs_out) *n_pairs_out = total;
-    cleanup();
 #undef TRY
-#undef TRYC
     return DYN_OK;
 }
 
@@ -784,21 +1014,41 @@ int nb_forces(dyn_nb_t h, const float* pos_dyn, const float* pos_w_o,
     const float3 ext = make_float3(cell_extent[0], cell_extent[1], cell_extent[2]);
     // the reference computes the reciprocal extent on the host in float32
     const float3 inv_ext = make_float3(1.0f / ext.x, 1.0f / ext.y, 1.0f / ext.z);
-    int blocks = (int)std::min<uint64_t>((h->n_pairs + NB_BLOCK - 1) / NB_BLOCK, NB_MAX_BLOCKS);
-    if (blocks < 1) blocks = 1;
+    // the flat entries but the water pairs of a built list, which are taken
+    // by molecule
+    const uint64_t n_flat = h->n_pairs - 10 * h->n_ww;
+    auto nblk = [](uint64_t n) {
+        return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + NB_BLOCK - 1) / NB_BLOCK, NB_MAX_BLOCKS));
+    };
+    const int blocks = nblk(n_flat);
     PosPtrs pp;
     ForcePtrs fp;
     for (int a = 0; a < 5; ++a) { pp.p[a] = h->d_pos[a]; fp.f[a] = h->d_f[a]; }
+    PairConsts pc{};
+    pc.ext = ext;
+    pc.inv_ext = inv_ext;
+    pc.half = make_float3(0.4999f * ext.x, 0.4999f * ext.y, 0.4999f * ext.z);
+    pc.rc = h->rc; pc.alpha = h->alpha; pc.ljc = h->ljc;
+    pc.ovr = override_bits;
     // the alchemical kernel runs when any installed pair is alchemical, as
     // force_nonbonded_gpu picks it (src/gpu_interface.rs:488-499)
     const AlchSched al = alch_schedule(lambda);
     const bool cpu = h->ljc > 0.f, alch = h->n_alch > 0;
     auto kern = cpu ? (alch ? nb_pair_kernel<true, true> : nb_pair_kernel<true, false>)
                     : (alch ? nb_pair_kernel<false, true> : nb_pair_kernel<false, false>);
-    kern<<<blocks, NB_BLOCK, 0, st>>>(pp, fp, h->d_pidx, h->d_plj, h->d_pqq, h->n_pairs, ext, inv_ext,
-                                      h->rc, h->alpha, h->ljc, override_bits, al, h->d_partials);
+    kern<<<blocks, NB_BLOCK, 0, st>>>(pp, fp, h->d_pidx, h->d_plj, h->d_pqq, n_flat, pc, al, h->d_partials);
     DYN_CUDA(cudaGetLastError());
-    nb_finalize_kernel<<<1, 256, 0, st>>>(h->d_partials, blocks, h->d_scalars);
+    int all_blocks = blocks;
+    if (h->n_ww) {
+        const uint32_t run = ww_run(h->n_ww);
+        const int wb = nblk((h->n_ww + run - 1) / run);
+        auto wk = cpu ? nb_ww_kernel<true> : nb_ww_kernel<false>;
+        wk<<<wb, NB_BLOCK, 0, st>>>(pp, fp, h->d_wwi, h->d_wwj, h->n_ww, run, pc,
+                                      h->d_partials + (size_t)NB_PART * blocks);
+        DYN_CUDA(cudaGetLastError());
+        all_blocks += wb;
+    }
+    nb_finalize_kernel<<<1, 256, 0, st>>>(h->d_partials, all_blocks, h->d_scalars);
     DYN_CUDA(cudaGetLastError());
     for (int a = 0; a < 5; ++a) {
         const size_t n3 = 3 * (size_t)h->n_of(a);

@@ -269,3 +269,62 @@ def test_invalid_arguments_raise(gpu_lib):
         gi.force_nonbonded_gpu(fp, pn, np.zeros((2, 3)), [np.zeros((0, 3))] * 4, [20.0] * 3,
                                lambda_alch=float("nan"))
     fp.close()
+
+
+@pytest.mark.parametrize("lj_cutoff", [0.0, CUTOFF])
+@pytest.mark.parametrize("overrides", [0, 1, 2])
+@pytest.mark.parametrize("make", [water_only, mixed, synth.config1], ids=["water", "mixed", "config1"])
+def test_built_list_equals_the_same_list_reversed(gpu_lib, make, overrides, lj_cutoff):
+    """A built list's water pairs are evaluated by molecule; the same entries
+    in another order go through the general kernel.  The 64-bit sums are
+    the same integers; virial and energy are float64 sums in another order
+    (1e-12 of their size; terms of both signs cancel by less than 1e3)."""
+    sysd = make()
+    fp, pn = _build(sysd, lj_cutoff=lj_cutoff)
+    na = len(sysd["atom_pos"])
+    if na:
+        pn.mark_alchemical(0, na // 2)
+    pos_dyn, pw = _positions(sysd)
+    ext = (sysd["box_hi"] - sysd["box_lo"]).astype(np.float32)
+    # some coordinates outside the box: images by whole extents
+    pw = {k: np.where(np.arange(len(p))[:, None] % 7 == 0, p + ext, p).astype(np.float32) for k, p in pw.items()}
+    lam = 0.3
+    got = gi.force_nonbonded_gpu(fp, pn, pos_dyn, pw, ext, overrides, lam)
+    flat = pn.get_pairs()
+    n = len(flat["tgt"])
+    fl = flat["flags"]
+    pairs = {"tgt": flat["tgt"], "src": flat["src"], "sigma": flat["sigma"], "eps": flat["eps"], "q_tgt": flat["qq"],
+             "q_src": np.ones(n, np.float32), "body_tgt": flat["body_tgt"], "body_src": flat["body_src"],
+             "scale_14": fl & 1, "calc_lj": (fl >> 1) & 1, "calc_coulomb": (fl >> 2) & 1, "symmetric": (fl >> 3) & 1,
+             "alch": (fl >> 4) & 1}
+    pairs = {k: np.ascontiguousarray(a[::-1]) for k, a in pairs.items()}
+    fp2 = gi.ForcesPositsGpu(na, len(sysd["water_pos"]), CUTOFF, ALPHA, lj_cutoff)
+    pn2 = gi.PerNeighborGpu(fp2, pairs)
+    want = gi.force_nonbonded_gpu(fp2, pn2, pos_dyn, pw, ext, overrides, lam)
+    np.testing.assert_array_equal(got[0], want[0])
+    for k in want[1]:
+        np.testing.assert_array_equal(got[1][k], want[1][k])
+    for a, b in zip(got[2:], want[2:]):
+        assert abs(a - b) <= 1e-9 * max(abs(b), 1.0)
+    fp.close()
+    fp2.close()
+
+
+def test_rebuilt_list_grows_and_shrinks(gpu_lib):
+    """The device areas of the build are kept between calls: a handle that
+    builds for dense, sparse and dense positions again gives what a new one
+    gives."""
+    sysd = mixed()
+    fp = gi.ForcesPositsGpu(len(sysd["atom_pos"]), len(sysd["water_pos"]), CUTOFF, ALPHA, CUTOFF)
+    args = (sysd["atom_q"], sysd["atom_sigma"], sysd["atom_eps"], sysd["box_lo"])
+    for scale in (1.0, 2.5, 0.9, 1.0):
+        p, w = sysd["atom_pos"] * np.float32(scale), sysd["water_pos"][:, 0] * np.float32(scale)
+        hi = sysd["box_hi"] * np.float32(scale)
+        a = gi.PerNeighborGpu.build(fp, p, w, *args, hi, SKIN, excl=sysd.get("excl"), pair14=sysd.get("pair14"))
+        fresh = gi.ForcesPositsGpu(fp.n_dyn, fp.n_water, CUTOFF, ALPHA, CUTOFF)
+        b = gi.PerNeighborGpu.build(fresh, p, w, *args, hi, SKIN, excl=sysd.get("excl"), pair14=sysd.get("pair14"))
+        ga, gb = a.get_pairs(), b.get_pairs()
+        for k in ga:
+            np.testing.assert_array_equal(ga[k], gb[k])
+        fresh.close()
+    fp.close()
