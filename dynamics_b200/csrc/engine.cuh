@@ -212,7 +212,7 @@ struct SysView {
     uint32_t* brick_sid;    // site codes (atom index, or DYN_SITE_WATER | 3 * water id + site)
     SiteRec* ovf_site;      // [n_sites_max]
     uint32_t* ovf_sid;
-    float* wsite_f;         // [nw*9] reciprocal force on H0, H1, M by water id, before corrections
+    float* wsite_f;         // [nw*9] reciprocal force on H0, H1, M by water id, before corrections (with them only)
     // box and scalars
     BoxDev* box;
     Scalars* sc;

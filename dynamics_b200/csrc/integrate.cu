@@ -128,6 +128,7 @@ DYN_KERNEL(, k_water_first, (, float dt), (, dt)) {
         if (id == INVALID_ID) continue;
         float3 o = xyz(v.wpos[4 * s]), h0 = xyz(v.wpos[4 * s + 1]), h1 = xyz(v.wpos[4 * s + 2]);
         float3 vo = xyz(v.wvel[3 * s]), vh0 = xyz(v.wvel[3 * s + 1]), vh1 = xyz(v.wvel[3 * s + 2]);
+        const float3 at_rebuild = xyz(v.wref[s]), at_prune = xyz(v.wprune[s]);
         const float hk = 0.5f * dt;
         vo = vo + xyz(v.wacc[3 * s]) * hk;
         vh0 = vh0 + xyz(v.wacc[3 * s + 1]) * hk;
@@ -154,7 +155,7 @@ DYN_KERNEL(, k_water_first, (, float dt), (, dt)) {
         int4* wf = reinterpret_cast<int4*>(v.wforce + 12 * (size_t)s);
 #pragma unroll
         for (int k = 0; k < 6; ++k) wf[k] = make_int4(0, 0, 0, 0);
-        const float3 d = min_image_rint(o - xyz(v.wref[s]), b), dp = min_image_rint(o - xyz(v.wprune[s]), b);
+        const float3 d = min_image_rint(o - at_rebuild, b), dp = min_image_rint(o - at_prune, b);
         const float d2 = dot3(d, d), dp2 = dot3(dp, dp);
         md = fmaxf(md, isfinite(d2) ? d2 : 1e30f);
         mdp = fmaxf(mdp, isfinite(dp2) ? dp2 : 1e30f);
@@ -508,10 +509,11 @@ __device__ double gamma_mt(double shape, uint64_t step, uint64_t seed) {
     return d;
 }
 
-DYN_KERNEL_T((bool ENERGY), (ENERGY), , k_finalize, (, float dt, bool thermo), (, dt, thermo)) {
-    // one warp per region, all regions' partials in flight at once; each
-    // region's sum has a fixed order
-    __shared__ double rs[NREGION][4];
+DYN_KERNEL_T((bool ENERGY), (ENERGY), __launch_bounds__(1024), k_finalize, (, float dt, bool thermo), (, dt, thermo)) {
+    // all regions' partials in flight at once, over 26 warps; each region's
+    // sum has a fixed order
+    constexpr int NFIN = 8;
+    __shared__ double rs[NREGION][4], part[32][4];
     // the thermostat's and barostat's random numbers depend only on the
     // step and the seed: two otherwise idle warps draw them while the
     // others reduce the partials
@@ -521,7 +523,7 @@ DYN_KERNEL_T((bool ENERGY), (ENERGY), , k_finalize, (, float dt, bool thermo), (
     const bool baro_on = thermo && v.barostat == DYN_BARO_CRESCALE && v.tau_p > 0.f;
     {
         const uint32_t wr = threadIdx.x >> 5;
-        const uint32_t w_csvr = NREGION % (blockDim.x >> 5), w_baro = (NREGION + 1) % (blockDim.x >> 5);
+        const uint32_t w_csvr = 30, w_baro = 31;
         const uint64_t step = v.sc->step;
         if (csvr_on && wr == w_csvr && (threadIdx.x & 31) == 0) {
             const double dof = (double)(v.thermo_dof > 2 ? v.thermo_dof : 2);
@@ -538,32 +540,50 @@ DYN_KERNEL_T((bool ENERGY), (ENERGY), , k_finalize, (, float dt, bool thermo), (
         }
     }
     {
+        // the regions' shares of the warps: the pair kernels' thousands of
+        // partials over several, so that no warp's chain of loads sets the
+        // time (one warp per region: 10 us at 2,368 partials)
+        constexpr int FIRST[NFIN + 1] = {0, 4, 12, 20, 21, 22, 24, 25, 26};
+        constexpr int REG[NFIN] = {REG_WW, REG_WS, REG_SS, REG_14, REG_BOND, REG_KICK_W, REG_KICK_A, REG_CONS};
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        for (int reg = w; reg < NREGION; reg += (int)(blockDim.x >> 5)) {
+        int k = 0;
+#pragma unroll
+        for (int j = 1; j < NFIN; ++j) k += w >= FIRST[j] ? 1 : 0;
+        int reg = REG[0], first = FIRST[0], last = FIRST[1];
+#pragma unroll
+        for (int j = 1; j < NFIN; ++j)
+            if (k == j) { reg = REG[j]; first = FIRST[j]; last = FIRST[j + 1]; }
+        if (w < FIRST[NFIN]) {
             double o[4] = {0.0, 0.0, 0.0, 0.0};
-            const bool used = reg == REG_WW || reg == REG_KICK_W ||
-                              (v.na && (reg == REG_SS || reg == REG_14 || reg == REG_BOND ||
-                                        reg == REG_KICK_A || reg == REG_CONS || (v.nw && reg == REG_WS)));
-            if (used) {
-                const double4* p = reinterpret_cast<const double4*>(v.partials) + (size_t)reg * v.max_blocks;
-                const uint32_t n = v.nb[reg];
-                uint32_t i = lane;
-                for (; i + 96 < n; i += 128) {
-                    const double4 a = p[i], b = p[i + 32], c = p[i + 64], d = p[i + 96];
-                    o[0] += a.x; o[1] += a.y; o[2] += a.z; o[3] += a.w;
-                    o[0] += b.x; o[1] += b.y; o[2] += b.z; o[3] += b.w;
-                    o[0] += c.x; o[1] += c.y; o[2] += c.z; o[3] += c.w;
-                    o[0] += d.x; o[1] += d.y; o[2] += d.z; o[3] += d.w;
-                }
-                for (; i < n; i += 32) {
-                    const double4 a = p[i];
-                    o[0] += a.x; o[1] += a.y; o[2] += a.z; o[3] += a.w;
-                }
+            const double4* p = reinterpret_cast<const double4*>(v.partials) + (size_t)reg * v.max_blocks;
+            const uint32_t n = v.nb[reg], step = 32u * (uint32_t)(last - first);
+            uint32_t i = lane + 32u * (uint32_t)(w - first);
+            for (; i + 3 * step < n; i += 4 * step) {
+                const double4 a = p[i], b = p[i + step], c = p[i + 2 * step], d = p[i + 3 * step];
+                o[0] += a.x; o[1] += a.y; o[2] += a.z; o[3] += a.w;
+                o[0] += b.x; o[1] += b.y; o[2] += b.z; o[3] += b.w;
+                o[0] += c.x; o[1] += c.y; o[2] += c.z; o[3] += c.w;
+                o[0] += d.x; o[1] += d.y; o[2] += d.z; o[3] += d.w;
+            }
+            for (; i < n; i += step) {
+                const double4 a = p[i];
+                o[0] += a.x; o[1] += a.y; o[2] += a.z; o[3] += a.w;
             }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) o[k] = warp_sum_d(o[k]);
+            for (int q = 0; q < 4; ++q) o[q] = warp_sum_d(o[q]);
             if (lane == 0)
-                for (int k = 0; k < 4; ++k) rs[reg][k] = o[k];
+                for (int q = 0; q < 4; ++q) part[w][q] = o[q];
+        }
+        __syncthreads();
+        if (threadIdx.x < 4 * NFIN) {
+            const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
+            double x = 0.0;
+            int reg2 = REG[0], f2 = FIRST[0], l2 = FIRST[1];
+#pragma unroll
+            for (int j = 1; j < NFIN; ++j)
+                if (r == j) { reg2 = REG[j]; f2 = FIRST[j]; l2 = FIRST[j + 1]; }
+            for (int j = f2; j < l2; ++j) x += part[j][q];
+            rs[reg2][q] = x;
         }
     }
     __syncthreads();
@@ -945,9 +965,8 @@ void launch_second_half(const Target& t, float dt) {
 
 void launch_finalize(const Target& t, float dt, bool energy, bool thermo) {
     auto one = [](const SysView&) { return 1; };
-    // 16 warps: one per partial-sum region
-    if (energy) t.launch(k_finalize<true>, k_finalize_batch<true>, one, 512, 0, dt, thermo);
-    else t.launch(k_finalize<false>, k_finalize_batch<false>, one, 512, 0, dt, thermo);
+    if (energy) t.launch(k_finalize<true>, k_finalize_batch<true>, one, 1024, 0, dt, thermo);
+    else t.launch(k_finalize<false>, k_finalize_batch<false>, one, 1024, 0, dt, thermo);
     if (!thermo) return;
     t.launch(k_scale, k_scale_batch,
              [](const SysView& v) {

@@ -540,16 +540,28 @@ __device__ __forceinline__ float3 gather_rec(const SysView& v, const SiteRec& r,
     return f3(-q * v.K[0] * b.inv_ext[0] * gx, -q * v.K[1] * b.inv_ext[1] * gy, -q * v.K[2] * b.inv_ext[2] * gz);
 }
 
-// A site's reciprocal force: atoms into the reciprocal cache (pass 0 stores,
-// later passes add), water sites into the per-site scratch for
-// k_gather_wfin.
+// Systems with Ewald corrections add each water's intra-molecular ones to its
+// gathered forces in float64 before they are rounded to fixed point
+// (k_gather_wfin); the others need no such pass.
+__host__ __device__ __forceinline__ bool water_corrections(const SysView& v) {
+    return (v.flags & DYN_FLAG_EWALD_CORRECTIONS) != 0u;
+}
+
+// A site's reciprocal force into the reciprocal cache (pass 0 stores, later
+// passes add), or, with water corrections, into the per-site scratch of
+// k_gather_wfin.  Storing straight into the cache saved that kernel (4 us of
+// a 50 us SPME branch at 512 waters).
 __device__ __forceinline__ void gather_out(const SysView& v, uint32_t sid, float3 f, int pass) {
-    if (sid & DYN_SITE_WATER) {
-        float* o = v.wsite_f + 3 * (size_t)(sid & ~DYN_SITE_WATER);
-        o[0] = f.x; o[1] = f.y; o[2] = f.z;
-        return;
-    }
     long long* c = v.arecip + 3 * (size_t)sid;
+    if (sid & DYN_SITE_WATER) {
+        const size_t e = 3 * (size_t)(sid & ~DYN_SITE_WATER);
+        if (water_corrections(v)) {
+            float* o = v.wsite_f + e;
+            o[0] = f.x; o[1] = f.y; o[2] = f.z;
+            return;
+        }
+        c = v.wrecip + e;
+    }
     if (pass == 0) {
         c[0] = fix_from_float(f.x); c[1] = fix_from_float(f.y); c[2] = fix_from_float(f.z);
     } else {
@@ -633,12 +645,12 @@ DYN_KERNEL(__launch_bounds__(GB_T), k_gather_brick, (, int pass), (, pass)) {
     }
 }
 
-// Water reciprocal forces by molecule, into the cache by original id: the
-// sites' gathered forces in float64 plus, with Ewald corrections on, the
-// intra-water exclusion corrections (H0-H1, H0-M, H1-M).  Pass 0 stores,
+// Water reciprocal forces by molecule, into the cache by original id, for
+// systems with Ewald corrections: the sites' gathered forces in float64 plus
+// the intra-water exclusion corrections (H0-H1, H0-M, H1-M).  Pass 0 stores,
 // later passes add.
 DYN_KERNEL(, k_gather_wfin, (, int pass), (, pass)) {
-    const bool corr = pass == 0 && (v.flags & DYN_FLAG_EWALD_CORRECTIONS);
+    const bool corr = pass == 0;
     double e_c = 0.0, w_c = 0.0;
     for (uint32_t s = bk.idx * blockDim.x + threadIdx.x; s < v.nw_cap; s += bk.cnt * blockDim.x) {
         const uint32_t id = v.wid[s];
@@ -746,7 +758,7 @@ DYN_KERNEL(, k_corr_atoms, (), ()) {
 // Energy and virial of one SPME pass (fixed-order sums), weighted into the
 // evaluation's totals; with an alchemical molecule the cross term
 // E_full - E_env - E_mol times dcoulomb_scale/dlambda goes to dH/dlambda.
-DYN_KERNEL(, k_recip_pass, (, int pass), (, pass)) {
+__device__ __forceinline__ void recip_pass(const SysView& v, int pass) {
     double x[2] = {0.0, 0.0};
     for (uint32_t i = threadIdx.x; i < v.nb[REG_PME]; i += blockDim.x) {
         const double* p = v.partials + ((size_t)REG_PME * v.max_blocks + i) * 4;
@@ -771,9 +783,13 @@ DYN_KERNEL(, k_recip_pass, (, int pass), (, pass)) {
     }
 }
 
-// The evaluation's reciprocal energy (with the self term), virial and
-// corrections into the cache the steps between SPME evaluations reuse.
+DYN_KERNEL(, k_recip_pass, (, int pass), (, pass)) { recip_pass(v, pass); }
+
+// The last pass's sums, then the evaluation's reciprocal energy (with the
+// self term), virial and corrections into the cache the steps between SPME
+// evaluations reuse.
 DYN_KERNEL(, k_recip_finalize, (), ()) {
+    recip_pass(v, v.alch_on ? 2 : 0);
     double x[4] = {0.0, 0.0, 0.0, 0.0};
     for (uint32_t i = threadIdx.x; i < v.nb[REG_CORR]; i += blockDim.x) {
         const double* p = v.partials + ((size_t)REG_CORR * v.max_blocks + i) * 4;
@@ -808,7 +824,7 @@ int pme_blocks(const SysView& v) {
     return gblocks(v, (uint64_t)v.K[0] * v.K[1] * (v.K[2] / 2 + 1));
 }
 // blocks of k_gather_wfin (which writes the REG_CORR partials)
-int gather_blocks(const SysView& v) { return v.nw ? gblocks(v, v.nw_cap) : 0; }
+int gather_blocks(const SysView& v) { return v.nw && water_corrections(v) ? gblocks(v, v.nw_cap) : 0; }
 
 // The brick layout of the grid and the per-brick capacity (cap, or by
 // default about twice the mean charged sites per brick plus 32, a multiple
@@ -826,7 +842,10 @@ void pme_bricks(SysView& v, uint32_t cap) {
     v.brick_cap = std::min(512u, cap ? cap : (2u * mean + 32u + 31u) / 32u * 32u);
 }
 
-int corr_blocks(const SysView& v) { return gblocks(v, (uint64_t)v.n14 + v.nexcl); }
+int corr_blocks(const SysView& v) {
+    const uint64_t n = (uint64_t)v.n14 + v.nexcl;
+    return n ? gblocks(v, n) : 0;
+}
 
 int pme_init(SysView& v, cufftHandle* plan_f, cufftHandle* plan_b, cudaStream_t st) {
     const size_t n = (size_t)v.K[0] * v.K[1] * v.K[2];
@@ -938,7 +957,9 @@ void launch_pme_gather(const Target& t, int pass) {
     // the molecule's own pass (2) holds no water
     t.launch(k_gather_wfin, k_gather_wfin_batch,
              [&](const SysView& v) { return on(v) && pass != 2 ? (int)v.nb[REG_CORR] : 0; }, GT, 0, pass);
-    t.launch(k_recip_pass, k_recip_pass_batch, [&](const SysView& v) { return on(v) ? 1 : 0; }, 256, 0, pass);
+    // the last pass of an evaluation is summed by k_recip_finalize
+    t.launch(k_recip_pass, k_recip_pass_batch,
+             [&](const SysView& v) { return on(v) && pass < (v.alch_on ? 2 : 0) ? 1 : 0; }, 256, 0, pass);
 }
 
 void launch_pme(const Target& t) {

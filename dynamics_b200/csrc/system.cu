@@ -159,8 +159,15 @@ static int link_streams(cudaStream_t from, cudaStream_t to, cudaEvent_t e) {
     return DYN_OK;
 }
 
+// A fork whose branch stays empty would leave edges around the water kernels
+// that keep them from following one another directly (2 us each).
+static bool has_atoms(const Target& T) {
+    return T.any([](const SysView& v) { return v.na != 0u; });
+}
+
 int enqueue_first_half(const Target& T, const Target& A, const Branches& br, bool fork, float dt) {
     int rc;
+    fork = fork && has_atoms(T);
     if (fork && (rc = link_streams(T.st, A.st, br.ev[0])) != DYN_OK) return rc;
     launch_first_half_water(T, dt);
     launch_first_half_atoms(fork ? A : T, dt);
@@ -171,9 +178,10 @@ int enqueue_first_half(const Target& T, const Target& A, const Branches& br, boo
 int enqueue_forces(const Target& T, const Target& A, const Target& P, const Branches& br, bool fork, bool spme,
                    bool energy) {
     int rc;
-    if (fork && (rc = link_streams(T.st, A.st, br.ev[2])) != DYN_OK) return rc;
+    const bool fa = fork && has_atoms(T);
+    if (fa && (rc = link_streams(T.st, A.st, br.ev[2])) != DYN_OK) return rc;
     if (fork && spme && (rc = link_streams(T.st, P.st, br.ev[3])) != DYN_OK) return rc;
-    const Target& a = fork ? A : T;
+    const Target& a = fa ? A : T;
     const Target& p = fork ? P : T;
     if (spme) {
         launch_pme(p);
@@ -183,13 +191,14 @@ int enqueue_forces(const Target& T, const Target& A, const Target& P, const Bran
     launch_pair14(a, energy);
     launch_bonded(a, energy);
     launch_pairs_water(T, energy);
-    if (fork && (rc = link_streams(A.st, T.st, br.ev[4])) != DYN_OK) return rc;
+    if (fa && (rc = link_streams(A.st, T.st, br.ev[4])) != DYN_OK) return rc;
     if (fork && spme && (rc = link_streams(P.st, T.st, br.ev[5])) != DYN_OK) return rc;
     return DYN_OK;
 }
 
 int enqueue_second_half(const Target& T, const Target& A, const Branches& br, bool fork, float dt) {
     int rc;
+    fork = fork && has_atoms(T);
     if (fork && (rc = link_streams(T.st, A.st, br.ev[6])) != DYN_OK) return rc;
     launch_second_half_water(T, dt);
     launch_second_half_atoms(fork ? A : T, dt);
@@ -828,7 +837,7 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     TRY(dev_alloc(h, &v.brick_sid, (size_t)v.n_bricks * v.brick_cap, false));
     TRY(dev_alloc(h, &v.ovf_site, v.n_sites_max, false));
     TRY(dev_alloc(h, &v.ovf_sid, v.n_sites_max, false));
-    TRY(dev_alloc(h, &v.wsite_f, 9 * (size_t)v.nw));
+    TRY(dev_alloc(h, &v.wsite_f, v.flags & DYN_FLAG_EWALD_CORRECTIONS ? 9 * (size_t)v.nw : 0));
     v.plan_f = (int)h->plan_f;
     v.plan_b = (int)h->plan_b;
     {
