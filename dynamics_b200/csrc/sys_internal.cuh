@@ -120,11 +120,10 @@ int count_graph_kernels(cudaGraph_t g, uint32_t* n);
 // rebuilt), synchronous.
 int evaluate_forces(dyn_sys_s* h);
 
-// The parts of a step, enqueued on T's stream; with fork (only while a graph
-// is being captured) the independent work goes to the side targets A and P
-// (same systems, the side streams of br) as parallel branches that join
-// back into T.  The launch order is the same either way, which a batch needs
-// (it records its block maps in launch order).
+// The parts of a step, enqueued on T's stream; with fork the independent work
+// goes to the side targets A and P (same systems, the side streams of br) as
+// parallel branches that join back into T.  The launch order is the same
+// either way, which a batch needs (it records its block maps in launch order).
 //   first half:  water drift/thermostat on T | atom drift + constraints on A
 //   forces:      water-water, water-atom on T | atom-atom, 1-4, bonded on A |
 //                SPME and its corrections on P (spme steps)

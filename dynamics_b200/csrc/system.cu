@@ -272,25 +272,26 @@ int capture_step(dyn_sys_s* h, float dt, bool spme, bool energy, cudaGraph_t* ou
 
 // Forces at the current coordinates (no integration); dt = 0 kicks set the
 // accelerations without changing velocities.
-void enqueue_forces(dyn_sys_s* h, bool force_rebuild) {
+int enqueue_forces(dyn_sys_s* h, bool force_rebuild) {
     const SysView& v = h->v;
     cudaStream_t st = h->stream;
     const Target T{&v, nullptr, st};
+    const Target S0{&v, nullptr, h->br.side[0]}, S1{&v, nullptr, h->br.side[1]};
     if (!force_rebuild) dyn::launch_displacement_check(T);
     dyn::launch_rebuild(T, force_rebuild);
     if (!force_rebuild) dyn::launch_prune(T, false);  // a rebuild writes the pruned lists too
     dyn::launch_gather_atoms(T);
-    dyn::launch_pairs(T, true);
-    dyn::launch_pair14(T, true);
-    dyn::launch_bonded(T, true);
-    dyn::launch_pme(T);
-    dyn::launch_corrections(T);
-    dyn::launch_second_half(T, 0.0f);
+    // the branches of a step, also outside a graph
+    int rc = dyn::enqueue_forces(T, S0, S1, h->br, true, true, true);
+    if (rc == DYN_OK) rc = dyn::enqueue_second_half(T, S0, h->br, true, 0.0f);
+    if (rc != DYN_OK) return rc;
     dyn::launch_finalize(T, 0.0f, true, false);
+    return DYN_OK;
 }
 
 int evaluate_forces_now(dyn_sys_s* h) {
-    enqueue_forces(h, true);
+    const int rc = enqueue_forces(h, true);
+    if (rc != DYN_OK) return rc;
     return dyn::read_scalars(h);
 }
 
@@ -883,7 +884,7 @@ extern "C" int dyn_sys_create(void* stream, const dyn_config_t* cfg, const dyn_s
     if (v.nw) TRY(dyn::pair_ww_setup(v));
     TRYC(cudaStreamSynchronize(h->stream));
     // prime: first list build and forces -> accelerations
-    enqueue_forces(h, true);
+    TRY(enqueue_forces(h, true));
     TRYC(cudaGetLastError());
     TRY(read_scalars(h));
 #undef TRY
@@ -949,39 +950,63 @@ extern "C" int dyn_sys_get_energies(dyn_sys_t h, dyn_energies_t* out) {
     return rc;
 }
 
+// Forces in home order and float64, [nw][O, H0, H1, M][3] by water id and
+// then [na][3]: components [lo, lo + n) of that sequence into out.
+__global__ void k_forces_out(const __grid_constant__ SysView v, double* __restrict__ out, size_t lo, size_t n) {
+    const uint32_t stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t t = first; t < 4u * v.nw_cap; t += stride) {
+        const uint32_t s = t >> 2, k = t & 3u, id = v.wid[s];
+        if (id == INVALID_ID) continue;
+        const size_t o = 12 * (size_t)id + 3 * k;
+        if (o + 3 <= lo || o >= lo + n) continue;
+        // the cache holds H0, H1, M
+        const long long* r = v.wrecip + 9 * (size_t)id + 3 * (k - 1u);
+        for (int c = 0; c < 3; ++c) {
+            if (o + c < lo || o + c >= lo + n) continue;
+            const long long x = v.wforce[12 * (size_t)s + 3 * k + c] + (k ? r[c] : 0);
+            out[o + c - lo] = (double)x * DYN_FIX_INV;
+        }
+    }
+    const size_t a0 = 12 * (size_t)v.nw;
+    for (uint32_t t = first; t < 3u * v.na; t += stride) {
+        const size_t o = a0 + t;
+        if (o < lo || o >= lo + n) continue;
+        out[o - lo] = (double)(v.aforce[t] + v.arecip[t]) * DYN_FIX_INV;
+    }
+}
+
+// One force evaluation.  The forces are put together and converted on the
+// device and copied once (three arrays, 76 bytes a water more and a pass over
+// them on one host core before; with the evaluation's kernels on parallel
+// branches 793 -> 441 us a call at 8,000 waters).  They pass through the partial sums of the regions that every evaluation rewrites
+// before it reads them (up to REG_CONS, which the first half of a step
+// leaves for the next evaluation), several times if they do not fit.
 extern "C" int dyn_sys_forces(dyn_sys_t h, double* f_atoms, double* f_water, dyn_energies_t* energies) {
     DYN_CHECK(h, DYN_ERR_INVALID, "dyn_sys_forces: NULL handle");
     const SysView& v = h->v;
-    enqueue_forces(h, false);
-    DYN_CUDA(cudaGetLastError());
-    int rc = read_scalars(h);
+    cudaStream_t st = h->stream;
+    int rc = enqueue_forces(h, false);
     if (rc) return rc;
-    if (f_atoms && v.na) {
-        std::vector<long long> a(3 * (size_t)v.na), r(3 * (size_t)v.na);
-        DYN_CUDA(cudaMemcpy(a.data(), v.aforce, a.size() * 8, cudaMemcpyDeviceToHost));
-        DYN_CUDA(cudaMemcpy(r.data(), v.arecip, r.size() * 8, cudaMemcpyDeviceToHost));
-        for (size_t k = 0; k < a.size(); ++k) f_atoms[k] = (double)(a[k] + r[k]) * DYN_FIX_INV;
+    DYN_CUDA(cudaGetLastError());
+    BoxDev bx;
+    if (energies) DYN_CUDA(cudaMemcpyAsync(&bx, v.box, sizeof(BoxDev), cudaMemcpyDeviceToHost, st));
+    if ((rc = read_scalars(h)) != DYN_OK) return rc;
+    const size_t room = (size_t)REG_CONS * v.max_blocks * 4, mid = 12 * (size_t)v.nw, end = mid + 3 * (size_t)v.na;
+    for (size_t lo = f_water ? 0 : mid, hi; lo < (f_atoms ? end : mid); lo = hi) {
+        hi = std::min(lo + room, f_atoms ? end : mid);
+        const uint32_t work = std::max(4u * v.nw_cap, 3u * v.na);
+        k_forces_out<<<(int)std::min<uint32_t>((work + 255) / 256, 148 * 8), 256, 0, st>>>(v, v.partials, lo, hi - lo);
+        DYN_CUDA(cudaGetLastError());
+        const size_t w1 = std::min(hi, mid);
+        if (lo < w1)
+            DYN_CUDA(cudaMemcpyAsync(f_water + lo, v.partials, (w1 - lo) * 8, cudaMemcpyDeviceToHost, st));
+        const size_t a0 = std::max(lo, mid);
+        if (a0 < hi)
+            DYN_CUDA(cudaMemcpyAsync(f_atoms + (a0 - mid), v.partials + (a0 - lo), (hi - a0) * 8,
+                                     cudaMemcpyDeviceToHost, st));
     }
-    if (f_water && v.nw) {
-        std::vector<long long> f(12 * (size_t)v.nw_cap), r(9 * (size_t)v.nw);
-        std::vector<uint32_t> wid(v.nw_cap);
-        DYN_CUDA(cudaMemcpy(f.data(), v.wforce, f.size() * 8, cudaMemcpyDeviceToHost));
-        DYN_CUDA(cudaMemcpy(r.data(), v.wrecip, r.size() * 8, cudaMemcpyDeviceToHost));
-        DYN_CUDA(cudaMemcpy(wid.data(), v.wid, wid.size() * 4, cudaMemcpyDeviceToHost));
-        for (uint32_t s = 0; s < v.nw_cap; ++s) {
-            const uint32_t id = wid[s];
-            if (id == INVALID_ID) continue;
-            // sites O, H0, H1, M; the cache holds H0, H1, M
-            for (int c = 0; c < 12; ++c) {
-                long long x = f[12 * (size_t)s + c];
-                if (c >= 3) x += r[9 * (size_t)id + (c - 3)];
-                f_water[12 * (size_t)id + c] = (double)x * DYN_FIX_INV;
-            }
-        }
-    }
+    DYN_CUDA(cudaStreamSynchronize(st));
     if (energies) {
-        BoxDev bx;
-        DYN_CUDA(cudaMemcpy(&bx, v.box, sizeof(BoxDev), cudaMemcpyDeviceToHost));
         fill_energies(h, energies);
         for (int k = 0; k < 3; ++k) energies->box[k] = bx.ext[k];
     }
@@ -1067,7 +1092,8 @@ extern "C" int dyn_sys_set_state(dyn_sys_t h, const float* atom_pos, const float
         DYN_CUDA(cudaMemcpy(v.wvel, w.data(), w.size() * sizeof(float4), cudaMemcpyHostToDevice));
     }
     // new coordinates: rebuild lists and re-prime forces/accelerations
-    enqueue_forces(h, true);
+    const int rc = enqueue_forces(h, true);
+    if (rc != DYN_OK) return rc;
     DYN_CUDA(cudaGetLastError());
     return read_scalars(h);
 }

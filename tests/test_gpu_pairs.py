@@ -73,3 +73,30 @@ def test_batch_members_of_other_cutoffs(gpu_lib):
             np.testing.assert_array_equal(got[k], want[k])
         alone.close()
     b.close()
+
+
+@pytest.mark.parametrize("n_side,mol_len", [(7, 5), (19, 5), (19, 0)])
+def test_forces_output(gpu_lib, n_side, mol_len):
+    """The forces handed to the host, at a size that passes through the
+    device's scratch at once and at one that takes two turns (6,314 waters a
+    turn): against the oracle; the same bits from a second call, whose energies
+    come from the partial sums the scratch shares, and for each output alone."""
+    from dynamics_b200 import _lib
+
+    sysd = mixed(n_side=n_side, mol_len=mol_len) if mol_len else water_only(n_side)
+    cfg = _cfg(sysd, "corrected")
+    st = md.MdState(sysd, cfg)
+    st.step(0.001, 3)
+    got = st.forces()
+    s = st.state()
+    ref = _oracle({**sysd, "water_pos": s["water_pos"], "atom_pos": s["atom_pos"]}, cfg, st)
+    assert _compare(got, ref) < FORCE_RTOL
+    again = st.forces()
+    for k in got:
+        np.testing.assert_array_equal(got[k], again[k])
+    for k in ("f_atoms", "f_water"):
+        part = np.full_like(got[k], np.nan)
+        a, w = (_lib.ptr(part), None) if k == "f_atoms" else (None, _lib.ptr(part))
+        _lib.check(_lib.lib().dyn_sys_forces(st.handle, a, w, None))
+        np.testing.assert_array_equal(part, got[k])
+    st.close()
