@@ -978,9 +978,10 @@ __global__ void k_forces_out(const __grid_constant__ SysView v, double* __restri
 // One force evaluation.  The forces are put together and converted on the
 // device and copied once (three arrays, 76 bytes a water more and a pass over
 // them on one host core before; with the evaluation's kernels on parallel
-// branches 793 -> 441 us a call at 8,000 waters).  They pass through the partial sums of the regions that every evaluation rewrites
-// before it reads them (up to REG_CONS, which the first half of a step
-// leaves for the next evaluation), several times if they do not fit.
+// branches 793 -> 441 us a call at 8,000 waters).  They pass through the
+// partial sums of the regions that every evaluation rewrites before it reads
+// them (up to REG_CONS, which the first half of a step leaves for the next
+// evaluation), several times if they do not fit.
 extern "C" int dyn_sys_forces(dyn_sys_t h, double* f_atoms, double* f_water, dyn_energies_t* energies) {
     DYN_CHECK(h, DYN_ERR_INVALID, "dyn_sys_forces: NULL handle");
     const SysView& v = h->v;
@@ -1496,8 +1497,15 @@ void energies_of(dyn_sys_s* h, dyn_energies_t* e) { fill_energies(h, e); }
 
 void set_batch_member(dyn_sys_s* h) {
     h->batch_member = true;
-    // the batch fills the GPU: no automatic group split
-    if (h->cfg.ww_split == 0) h->v.ww_split = 1;
+    // the batch fills the GPU: no automatic group split, and chunks for 3 CTAs
+    // per SM although the batch form of the kernel runs 2: the shared memory
+    // left over lets the SPME branch run beside it (64 systems of 512 to 8,000
+    // waters: 1241 us a step with the larger chunks, 1168 with these, 1290
+    // with 256 waters; one system of 8,000 waters alone 108 and 112)
+    if (h->cfg.ww_split == 0) {
+        h->v.ww_split = 1;
+        h->v.union_chunk = ww_chunk_for(h->v, &h->cfg, 3);
+    }
     set_block_counts(h->v);
 }
 }  // namespace dyn

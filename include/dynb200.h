@@ -326,8 +326,10 @@ typedef struct {
                              * entries in the water-water kernel (1..8);
                              * 0 = automatic: more than 1 only for a system
                              * stepped alone with fewer groups than the GPU
-                             * has SMs; batch members get 1.  A tuning knob:
-                             * results change only at rounding level.       */
+                             * has SMs; batch members get 1, and smaller
+                             * automatic chunks (ww_union_chunk).  A tuning
+                             * knob: results change only at rounding level; a
+                             * member set to 1 or more steps as alone.      */
 } dyn_config_t;
 
 typedef struct {
