@@ -41,6 +41,7 @@ struct dyn_nb_s {
     size_t off[5] = {}, n_comp = 0;
     float* d_pos = nullptr;
     long long* d_f = nullptr;      // fixed-point forces, then virial, energy, dH/dlambda (double)
+    float4* d_sphere = nullptr;    // [n_water] centre and radius of each water's sites
     double* d_partials = nullptr;  // [2 * NB_MAX_BLOCKS * NB_PART]
     uint64_t n_alch = 0;           // installed pairs with the alchemical bit
     // device memory of dyn_nb_build_pairs, kept between calls: its inputs and
@@ -252,31 +253,84 @@ __global__ void __launch_bounds__(NB_BLOCK) nb_pair_kernel(
     write_nb_partials(w_acc, e_acc, h_acc, partials);
 }
 
+// Bounding spheres of the waters: the midpoint of the hydrogens and the
+// largest distance of a site from it, with room for the rounding of this and
+// of the distances compared with it.  Waters of any shape, also one broken
+// over the box's faces, whose sphere is then as large as the box.
+__global__ void nb_sphere_kernel(PosPtrs pos, uint32_t n, float3 ext, float4* __restrict__ sphere) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float3 h0 = ld_pos(pos.p, 3, i), h1 = ld_pos(pos.p, 4, i);
+        const float3 c = (h0 + h1) * 0.5f;
+        float r2 = 0.f, big = fmaxf(ext.x, fmaxf(ext.y, ext.z));
+        bool finite = true;
+        for (int b = 1; b < 5; ++b) {
+            const float3 x = ld_pos(pos.p, b, i), d = x - c;
+            const float d2 = dot3(d, d);
+            finite = finite && isfinite(d2);
+            r2 = fmaxf(r2, d2);
+            big = fmaxf(big, fmaxf(fabsf(x.x), fmaxf(fabsf(x.y), fabsf(x.z))));
+        }
+        sphere[i] = make_float4(c.x, c.y, c.z, finite ? sqrtf(r2) * 1.000001f + 2e-6f * big : INFINITY);
+    }
+}
+
 // The water-water part of a list in setup_pairs' order, from its
 // molecule pairs (8 bytes each) instead of their ten flat entries (200 bytes).
-// A thread takes run consecutive molecule pairs, which mostly share the
-// first water: every site pair is evaluated and rounded to fixed point as by
-// the general kernel, the first water's forces are summed in 64-bit registers
-// until it changes and the second's per molecule pair, so the sums are the
-// same integers.  Bound by issue (pairs beyond the cutoff cost their distance
-// only).  1.4 M molecule pairs of 7,800 waters (13 A list, 9 A cutoff): 148 us,
-// against 942 us for their 14 M flat entries with six reductions each.  Runs
-// of 8 where that leaves four waves of threads, shorter ones below (89,000
-// molecule pairs in runs of 8 left most of the SMs without work: 58 us).
-constexpr uint64_t WW_RUN = 8, WW_THREADS = 148 * 1024;
+// A warp takes 32 run consecutive molecule pairs, which mostly share the
+// first water, and its lanes equal contiguous shares of them: every site pair
+// is evaluated and rounded to fixed point as by the general kernel, the first
+// water's forces are summed in 64-bit registers until it changes and the
+// second's per molecule pair, so the sums are the same integers.  With an LJ
+// cutoff (CPU_SEM) no force reaches beyond the cutoffs, and only the molecule
+// pairs whose bounding spheres come that near are shared out: bound by issue,
+// and two thirds of a list with skin lie beyond, but a warp in which one lane's
+// pair is in reach evaluates for all.  1.4 M molecule pairs of 7,800 waters
+// (13 A list, 9 A cutoff): 116 us, 176 without the selection, 942 as 14 M flat
+// entries with six reductions each.  Runs of 16 where that leaves two waves of
+// threads, shorter ones below (89,000 molecule pairs in runs of 8 left most of
+// the SMs without work: 58 us).
+constexpr uint64_t WW_RUN = 16, WW_THREADS = 148 * 1024;
 inline uint32_t ww_run(uint64_t n) { return (uint32_t)std::max<uint64_t>(1, std::min(WW_RUN, n / WW_THREADS)); }
 
 template <bool CPU_SEM>
 __global__ void __launch_bounds__(NB_BLOCK) nb_ww_kernel(PosPtrs pos, ForcePtrs out, const uint32_t* __restrict__ wi,
                                                          const uint32_t* __restrict__ wj, uint64_t n, uint32_t run,
-                                                         PairConsts c, double* __restrict__ partials) {
+                                                         const float4* __restrict__ sphere, PairConsts c,
+                                                         double* __restrict__ partials) {
+    __shared__ uint16_t near[CPU_SEM ? NB_BLOCK * WW_RUN : 1];  // a warp's selected pairs
     // sites in setup_pairs' order O, M, H0, H1 = bodies 1..4
     const float q[4] = {0.f, OPC_Q_EP, OPC_Q_H, OPC_Q_H};
     const AlchSched none{1.f, 0.f, 0.f, 0.f};
     double w_acc = 0.0;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, piece = 32u * run;
+    uint16_t* sel = near + (CPU_SEM ? warp * piece : 0u);
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * run;
-    for (uint64_t k0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * run; k0 < n; k0 += stride) {
-        const uint64_t k1 = k0 + run < n ? k0 + run : n;
+    // k0: the warp's first pair, the same in all its lanes
+    for (uint64_t k0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + warp) * piece; k0 < n; k0 += stride) {
+        uint32_t cnt = k0 + piece < n ? piece : (uint32_t)(n - k0);
+        if (CPU_SEM) {
+            const float reach = fmaxf(c.rc, c.ljc);
+            uint32_t m = 0;
+            for (uint32_t t = lane; t < piece; t += 32) {
+                bool in = false;
+                if (t < cnt) {
+                    const float4 a = sphere[wi[k0 + t]], b = sphere[wj[k0 + t]];
+                    float3 d = f3(a.x - b.x, a.y - b.y, a.z - b.z);
+                    d.x -= rintf(d.x * c.inv_ext.x) * c.ext.x;
+                    d.y -= rintf(d.y * c.inv_ext.y) * c.ext.y;
+                    d.z -= rintf(d.z * c.inv_ext.z) * c.ext.z;
+                    const float d2 = dot3(d, d), l = reach + a.w + b.w;
+                    // not finite: evaluated, as without the selection
+                    in = !(d2 > l * l) || !isfinite(d2);
+                }
+                const uint32_t mask = __ballot_sync(0xffffffffu, in);
+                if (in) sel[m + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)t;
+                m += __popc(mask);
+            }
+            cnt = m;
+            __syncwarp();
+        }
+        const uint32_t t0 = lane * cnt / 32u, t1 = (lane + 1u) * cnt / 32u;
         uint32_t cur = 0xFFFFFFFFu;
         float3 pi[4];
         long long fi[12];
@@ -289,7 +343,8 @@ __global__ void __launch_bounds__(NB_BLOCK) nb_ww_kernel(PosPtrs pos, ForcePtrs 
                     for (int x = 0; x < 3; ++x)
                         if (fi[3 * s + x]) fix_atomic_add(out.f[s + 1] + 3 * (size_t)cur + x, fi[3 * s + x]);
         };
-        for (uint64_t k = k0; k < k1; ++k) {
+        for (uint32_t t2 = t0; t2 < t1; ++t2) {
+            const uint64_t k = k0 + (CPU_SEM ? (uint32_t)sel[t2] : t2);
             const uint32_t i = wi[k], j = wj[k];
             if (i != cur) {
                 flush();
@@ -330,6 +385,7 @@ __global__ void __launch_bounds__(NB_BLOCK) nb_ww_kernel(PosPtrs pos, ForcePtrs 
             }
         }
         flush();
+        __syncwarp();  // the selection is refilled
     }
     write_nb_partials(w_acc, 0.0, 0.0, partials);
 }
@@ -706,6 +762,7 @@ extern "C" int dyn_nb_create(void* stream, uint32_t n_dyn, uint32_t n_water, flo
     if (rc == DYN_OK) rc = dalloc(&h->d_f, h->n_comp + NB_PART);
     if (rc == DYN_OK) rc = halloc(&h->h_pos, h->n_comp);
     if (rc == DYN_OK) rc = halloc(&h->h_f, h->n_comp + NB_PART);
+    if (rc == DYN_OK) rc = dalloc(&h->d_sphere, n_water);
     if (rc == DYN_OK) rc = dalloc(&h->d_partials, 2 * NB_PART * NB_MAX_BLOCKS);
     if (rc != DYN_OK) {
         dyn_nb_destroy(h);
@@ -720,7 +777,7 @@ extern "C" int dyn_nb_destroy(dyn_nb_t h) {
     if (h->stream) cudaStreamSynchronize(h->stream); else cudaDeviceSynchronize();
     cudaFree(h->d_pos); cudaFree(h->d_f);
     cudaFreeHost(h->h_pos); cudaFreeHost(h->h_f);
-    cudaFree(h->d_partials);
+    cudaFree(h->d_sphere); cudaFree(h->d_partials);
     cudaFree(h->d_pidx); cudaFree(h->d_plj); cudaFree(h->d_pqq);
     cudaFree(h->scratch.p); cudaFree(h->lists.p);
     delete h;
@@ -1054,7 +1111,9 @@ int nb_forces(dyn_nb_t h, const float* pos_dyn, const float* pos_w_o,
         const uint32_t run = ww_run(h->n_ww);
         const int wb = nblk((h->n_ww + run - 1) / run);
         auto wk = cpu ? nb_ww_kernel<true> : nb_ww_kernel<false>;
-        wk<<<wb, NB_BLOCK, 0, st>>>(pp, fp, h->d_wwi, h->d_wwj, h->n_ww, run, pc,
+        if (cpu)
+            nb_sphere_kernel<<<nblk(h->n_water), NB_BLOCK, 0, st>>>(pp, h->n_water, ext, h->d_sphere);
+        wk<<<wb, NB_BLOCK, 0, st>>>(pp, fp, h->d_wwi, h->d_wwj, h->n_ww, run, h->d_sphere, pc,
                                       h->d_partials + (size_t)NB_PART * blocks);
         DYN_CUDA(cudaGetLastError());
         all_blocks += wb;

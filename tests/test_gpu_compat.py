@@ -328,3 +328,48 @@ def test_rebuilt_list_grows_and_shrinks(gpu_lib):
             np.testing.assert_array_equal(ga[k], gb[k])
         fresh.close()
     fp.close()
+
+
+@pytest.mark.parametrize("lj_cutoff", [0.0, 5.5, CUTOFF + 1.5])
+@pytest.mark.parametrize("odd", ["none", "broken", "outside", "stretched", "nan"])
+def test_water_pairs_selected_by_reach(gpu_lib, odd, lj_cutoff):
+    """A built list's water pairs are evaluated where their bounding spheres
+    come within the cutoffs: the same integers as the general kernel's for
+    waters broken over the box's faces, outside the box, out of shape, not
+    finite, and for either cutoff the larger."""
+    sysd = water_only()
+    ext = (sysd["box_hi"] - sysd["box_lo"]).astype(np.float32)
+    fp, pn = _build(sysd, lj_cutoff=lj_cutoff)
+    pos_dyn, pw = _positions(sysd)
+    pw = {k: np.array(p, np.float32) for k, p in pw.items()}  # O, M, H0, H1 = 1..4
+    w = np.arange(0, len(sysd["water_pos"]), 7)
+    if odd == "broken":
+        pw[4][w, 0] += ext[0]
+        pw[3][w[1:], 2] -= ext[2]
+    elif odd == "outside":
+        for p in pw.values():
+            p[w] += 3 * ext
+    elif odd == "stretched":
+        pw[3][w] += np.float32(4.0)
+        pw[1][w[::2]] -= np.float32(2.5)
+    elif odd == "nan":
+        pw[2][w[3]] = np.nan
+        pw[1][w[5], 1] = np.inf
+    got = gi.force_nonbonded_gpu(fp, pn, pos_dyn, pw, ext)
+    flat = pn.get_pairs()
+    n = len(flat["tgt"])
+    fl = flat["flags"]
+    pairs = {"tgt": flat["tgt"], "src": flat["src"], "sigma": flat["sigma"], "eps": flat["eps"], "q_tgt": flat["qq"],
+             "q_src": np.ones(n, np.float32), "body_tgt": flat["body_tgt"], "body_src": flat["body_src"],
+             "scale_14": fl & 1, "calc_lj": (fl >> 1) & 1, "calc_coulomb": (fl >> 2) & 1, "symmetric": (fl >> 3) & 1,
+             "alch": (fl >> 4) & 1}
+    pairs = {k: np.ascontiguousarray(a[::-1]) for k, a in pairs.items()}
+    fp2 = gi.ForcesPositsGpu(fp.n_dyn, fp.n_water, CUTOFF, ALPHA, lj_cutoff)
+    want = gi.force_nonbonded_gpu(fp2, gi.PerNeighborGpu(fp2, pairs), pos_dyn, pw, ext)
+    for k in want[1]:
+        np.testing.assert_array_equal(got[1][k], want[1][k])
+    # the virial sums the same float64 terms in another order
+    if odd != "nan":
+        assert abs(got[2] - want[2]) <= 1e-9 * max(abs(want[2]), 1.0)
+    fp.close()
+    fp2.close()
